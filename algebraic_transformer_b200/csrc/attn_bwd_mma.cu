@@ -175,18 +175,18 @@ __global__ void __launch_bounds__(NTHREADS) attn_bwd_dq_kernel(const AttnBwdPara
   const __nv_bfloat16* kb = p.k + b * p.ks.b + h * p.ks.h;
   const __nv_bfloat16* vb = p.v + b * p.vs.b + h * p.vs.h;
   const __nv_bfloat16* ob = p.o + b * p.os.b + h * p.os.h;
-  const __nv_bfloat16* dob = p.d_o + b * p.os.b + h * p.os.h;
+  const __nv_bfloat16* dob = p.d_o + b * p.gs.b + h * p.gs.h;
   const int64_t bh = int64_t(b) * p.H + h;
 
   stage_tile<D>(qb, p.qs.t, q0, p.Tq, sQ);
-  stage_tile<D>(dob, p.os.t, q0, p.Tq, sdO);
+  stage_tile<D>(dob, p.gs.t, q0, p.Tq, sdO);
   // delta_i = dO_i . o_i: two threads per row, half of the columns each
   {
     const int r = threadIdx.x >> 1, half = threadIdx.x & 1;
     float d = 0.f;
     if (q0 + r < p.Tq) {
       const __nv_bfloat16* orow = ob + int64_t(q0 + r) * p.os.t + half * (D / 2);
-      const __nv_bfloat16* drow = dob + int64_t(q0 + r) * p.os.t + half * (D / 2);
+      const __nv_bfloat16* drow = dob + int64_t(q0 + r) * p.gs.t + half * (D / 2);
 #pragma unroll
       for (int cv = 0; cv < D / 16; ++cv) {
         const uint4 a = *reinterpret_cast<const uint4*>(orow + cv * 8), c = *reinterpret_cast<const uint4*>(drow + cv * 8);
@@ -300,7 +300,7 @@ __global__ void __launch_bounds__(NTHREADS) attn_bwd_dkv_kernel(const AttnBwdPar
   const __nv_bfloat16* qb = p.q + b * p.qs.b + h * p.qs.h;
   const __nv_bfloat16* kb = p.k + b * p.ks.b + h * p.ks.h;
   const __nv_bfloat16* vb = p.v + b * p.vs.b + h * p.vs.h;
-  const __nv_bfloat16* dob = p.d_o + b * p.os.b + h * p.os.h;
+  const __nv_bfloat16* dob = p.d_o + b * p.gs.b + h * p.gs.h;
   const int64_t bh = int64_t(b) * p.H + h;
 
   stage_tile<D>(kb, p.ks.t, k0, p.Tk, sK);
@@ -324,7 +324,7 @@ __global__ void __launch_bounds__(NTHREADS) attn_bwd_dkv_kernel(const AttnBwdPar
     const int q0 = qt * BM;
     __nv_bfloat16* dst = sQO + stage * 2 * TILE;
     stage_tile_async<D>(qb, p.qs.t, q0, p.Tq, dst);
-    stage_tile_async<D>(dob, p.os.t, q0, p.Tq, dst + TILE);
+    stage_tile_async<D>(dob, p.gs.t, q0, p.Tq, dst + TILE);
     if (threadIdx.x < BM) {
       const bool live = q0 + int(threadIdx.x) < p.Tq;
       s_stat[stage][threadIdx.x] = live ? p.stat[bh * p.Tq + q0 + threadIdx.x] : 0.f;

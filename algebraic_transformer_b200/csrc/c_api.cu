@@ -490,6 +490,7 @@ int alg_attn_bwd(const alg_attn_bwd_args* a, void* stream_) {
   p.ks = strides_or_dense(a->k_stride, a->H, a->Tk, a->D);
   p.vs = strides_or_dense(a->v_stride, a->H, a->Tk, a->D);
   p.os = strides_or_dense(a->o_stride, a->H, a->Tq, a->D);
+  p.gs = p.os;
   if (!strides_ok(p.qs, ALG_BF16) || !strides_ok(p.ks, ALG_BF16) || !strides_ok(p.vs, ALG_BF16) || !strides_ok(p.os, ALG_BF16) ||
       !aligned16(a->q) || !aligned16(a->k) || !aligned16(a->v) || !aligned16(a->o) || !aligned16(a->d_o) ||
       !aligned16(a->dq) || !aligned16(a->dk) || !aligned16(a->dv)) {

@@ -121,7 +121,7 @@ struct AttnBwdParams {
   const __nv_bfloat16* k;
   const __nv_bfloat16* v;
   const __nv_bfloat16* o;
-  const __nv_bfloat16* d_o;  // strides of o
+  const __nv_bfloat16* d_o;
   const float* stat;         // (B, H, Tq) saved by the forward
   const int* stat_kind;      // device: ALG_VARIANT_NOSHIFT / ALG_VARIANT_SHIFT, as the forward wrote it
   const float* sink;         // (H) or nullptr
@@ -136,12 +136,13 @@ struct AttnBwdParams {
   float n_scale, n_f;        // n * scale, n
   int causal;
   Strides3 qs, ks, vs, os;
+  Strides3 gs;               // of d_o
   int* status;               // device word for ALG_DEV_TIMEOUT, or nullptr
   int force_mma;             // 1: stay on the mma.sync kernels whatever the shape
 };
 // Dispatcher (attn_bwd_mma.cu): tcgen05 kernels when the shape fits them, else mma.sync.
 int launch_attn_bwd(const AttnBwdParams& p, cudaStream_t stream);
-// attn_bwd_sm100.cu: causal, Tq == Tk a multiple of 128, head_dim 64 or 128
+// attn_bwd_sm100.cu: causal self-attention (Tq == Tk) of any length, head_dim 64 or 128
 bool attn_bwd_tcgen05_supports(const AttnBwdParams& p);
 int launch_attn_bwd_tcgen05(const AttnBwdParams& p, cudaStream_t stream);
 
