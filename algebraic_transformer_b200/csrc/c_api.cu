@@ -538,7 +538,7 @@ int alg_head_bwd_dz(const alg_head_bwd_args* a, void* stream_) {
 size_t alg_decode_workspace_bytes(const alg_decode_args* a) {
   if (a == nullptr) return 0;
   // the splits' partial states, then one arrival word per (batch, head)
-  return align256(size_t(a->B) * a->H * decode_splits(a->B, a->H, a->Tk) * (a->D + 2) * sizeof(float)) + size_t(a->B) * a->H * 8;
+  return align256(size_t(a->B) * a->H * decode_splits(a->D, a->B, a->H, a->Tk) * (a->D + 2) * sizeof(float)) + size_t(a->B) * a->H * 8;
 }
 
 int alg_attn_decode(const alg_decode_args* a, void* stream) {
@@ -565,8 +565,8 @@ int alg_attn_decode(const alg_decode_args* a, void* stream) {
     set_error("decode: rows must start on 16-byte boundaries");
     return ALG_ERR_INVALID;
   }
-  p.splits = decode_splits(a->B, a->H, a->Tk);
-  p.keys_per_split = decode_keys_per_split(a->B, a->H, a->Tk);
+  p.splits = decode_splits(a->D, a->B, a->H, a->Tk);
+  p.keys_per_split = decode_keys_per_split(a->D, a->B, a->H, a->Tk);
   p.status = nullptr;
   p.part = static_cast<float*>(a->workspace);
   if (!aligned16(a->workspace)) { set_error("decode: workspace must be 16-byte aligned"); return ALG_ERR_INVALID; }

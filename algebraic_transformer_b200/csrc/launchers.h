@@ -204,8 +204,8 @@ struct DecodeParams {
   unsigned long long call;        // this call's number (unique per process): stale words of other calls read as zero arrivals
   int* status;
 };
-int decode_splits(int B, int H, int Tk);
-int decode_keys_per_split(int B, int H, int Tk);
+int decode_splits(int D, int B, int H, int Tk);
+int decode_keys_per_split(int D, int B, int H, int Tk);
 int launch_decode(const DecodeParams& p, cudaStream_t stream);
 
 // ---- Alg-CE head --------------------------------------------------------------------

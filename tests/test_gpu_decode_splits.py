@@ -1,0 +1,47 @@
+"""Decode at the sizes where its grid rule turns or a ring slot, a tile or a split is not full: one key, one tile and one
+key more, one CTA per head and several, one and two CTAs per SM, more heads than CTAs fit."""
+
+import pytest
+import torch
+
+import algebraic_transformer_b200 as A
+from oracle import algebraic_ref as R
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def rel_l2(a, b):
+    a, b = a.detach().double().cpu(), b.detach().double().cpu()
+    return float((a - b).norm() / b.norm().clamp_min(1e-30))
+
+
+def randn(shape, seed, dtype=torch.float32, scale=1.0):
+    return (torch.randn(shape, generator=torch.Generator().manual_seed(seed)) * scale).to(dtype)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("B,H,Tk", [(1, 1, 1), (1, 1, 33), (13, 23, 65), (32, 12, 200), (2, 74, 129), (10, 15, 385), (1, 2, 20000)])
+def test_decode_splits(B, H, Tk, D):
+    q, k, v = (randn((B, H, n, D), 31 + i, torch.bfloat16) for i, n in enumerate((1, Tk + 3, Tk)))
+    k = k.to(DEV)[:, :, :Tk]                                       # a cache with room to grow
+    for sink in (randn((H,), 34, scale=0.5), None):
+        want = R.asinh_attention(q, k.cpu(), v, n=16, c=8.0, sink_logit=sink, causal=False)
+        got = A.decode_attention(q.to(DEV), k, v.to(DEV), None if sink is None else sink.to(DEV), n=16, c=8.0)
+        assert rel_l2(got, want) < 5e-3                            # the output's bf16 rounding: 2^-9 an element at most
+        again = A.decode_attention(q.to(DEV), k, v.to(DEV), None if sink is None else sink.to(DEV), n=16, c=8.0)
+        assert torch.equal(got, again)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_decode_extremes(D):
+    """Scores far apart (the running maximum moves, weights underflow) and an infinite value."""
+    q, k, v = (randn((1, 2, n, D), 41 + i, torch.bfloat16) for i, n in enumerate((1, 700, 700)))
+    k = (k.float() * torch.logspace(-3, 3, 700)[None, None, :, None]).bfloat16()
+    want = R.asinh_attention(q, k, v, n=16, c=8.0, causal=False)
+    args = [t.to(DEV) for t in (q, k, v)]
+    assert rel_l2(A.decode_attention(*args, n=16, c=8.0), want) < 5e-3
+    args[2][0, 0, 5, 3] = float("inf")
+    args[1][0, 0, 5] = args[0][0, 0, 0]                            # a key with weight
+    got = A.decode_attention(*args, n=16, c=8.0).float()
+    assert got[0, 0, 0, 3] == float("inf") and torch.isfinite(got[0, 1]).all() and torch.isfinite(got[0, 0, 0, :3]).all()
