@@ -160,18 +160,32 @@ __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wa
 
 // Launch `kern` so that it may start before the kernel ahead of it in `stream` has finished
 // (programmatic dependent launch); the kernel itself calls griddep_wait() before it touches
-// anything the earlier kernel writes.
+// anything the earlier kernel writes.  `cluster` CTAs form a thread-block cluster.
+template <typename... Formal, typename... Actual>
+inline cudaError_t launch_dependent_cluster(int cluster, void (*kern)(Formal...), dim3 grid, dim3 block, size_t smem,
+                                            cudaStream_t stream, Actual&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  int n = 0;
+  static const bool plain = getenv("ALG_NO_PDL") != nullptr;      // measurement aid: ordinary stream order
+  if (!plain) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (cluster > 1) {
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = unsigned(cluster);
+    attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
+    ++n;
+  }
+  cfg.attrs = attr; cfg.numAttrs = n;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<Formal>(args)...);
+}
 template <typename... Formal, typename... Actual>
 inline cudaError_t launch_dependent(void (*kern)(Formal...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                                     Actual&&... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  static const bool plain = getenv("ALG_NO_PDL") != nullptr;      // measurement aid: ordinary stream order
-  cfg.attrs = attr; cfg.numAttrs = plain ? 0 : 1;
-  return cudaLaunchKernelEx(&cfg, kern, static_cast<Formal>(args)...);
+  return launch_dependent_cluster(1, kern, grid, block, smem, stream, static_cast<Actual&&>(args)...);
 }
 
 }  // namespace alg

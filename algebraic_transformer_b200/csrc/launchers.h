@@ -8,6 +8,21 @@
 
 namespace alg {
 
+// CTAs that share an accumulator tile in the GEMM kernels (projections, head): pairs (256-row tiles, each CTA
+// loading half of the weight rows, a third less operand traffic) where they take no more rounds of tiles than
+// single CTAs (128-row tiles) and a CTA has at least 64 ring steps to go: a pair starts and ends about 2 us later than a
+// single CTA, which has to be won back.  `row_blocks` 128-row blocks times `columns` tiles, or runs of tiles, of `steps`
+// ring steps beside each other.  Measured, single -> pairs: QKV 8192 x 768 (48 steps) 26.9 -> 28.6 us, 16384 x 1536 (768)
+// 177 -> 158; GLU 8192 x 768 (84) 41.6 -> 40.5, 16384 x 1536 (1392) 310 -> 272; down 16384 x 2048 x 768 (96) 46.2 -> 43.4,
+// out 16384 x 768 x 768 (36) 20.6 -> 22.8; head 8192 x 768 x 50304 441 -> 414, its gradient kernel 751 -> 659, head of 613
+// rows (5 blocks: a sixth of the pairs' work is padding) 45.5 -> 48.4.
+inline int pair_size(int row_blocks, int columns, int steps) {
+  const int64_t sms = sm_count(), pairs = sms / 2;
+  const int64_t single = (int64_t(row_blocks) * columns + sms - 1) / sms;
+  const int64_t paired = (int64_t((row_blocks + 1) / 2) * columns + pairs - 1) / pairs;
+  return paired <= single && single * steps >= 64 ? 2 : 1;
+}
+
 // ---- qk_prep.cu ---------------------------------------------------------------------
 struct PrepParams {
   const void* x;

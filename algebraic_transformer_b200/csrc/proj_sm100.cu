@@ -11,7 +11,7 @@
 //        statistic (src/algebraic/kernels/fused_head.py:120-156), written as bf16 for the two
 //        library GEMMs dh = dz . E and dE = dz^T . h that follow, as the reference does.
 //   RESID out = resid + x . W^T (the block's out- and down-projection with its residual add,
-//        src/algebraic/model.py:183, 193: the product rounded to bf16, then a bf16 add), and per
+//        src/algebraic/model.py:183, 193: added in fp32, rounded to bf16 once), and per
 //        row the sum of squares of what was written, as one partial per 128 or 64 output columns:
 //        the RMS normalisation that follows in the reference (model.py:141-143) is then carried
 //        by the NEXT projection, which multiplies its accumulator rows by tau = rsqrt(mean + eps)
@@ -23,8 +23,8 @@
 //        128 output features; gate and up never reach HBM.
 //
 // The main loop is the persistent, warp-specialised GEMM of head_sm100.cu: warp 0 (one lane)
-// feeds a 4-stage shared-memory ring with TMA (128x64 activation tiles, 256x64 weight tiles,
-// 128-byte swizzle), warp 1 (one lane) issues tcgen05.mma 128x256x16 into one of two 256-column
+// feeds a shared-memory ring with TMA (128x64 activation tiles, 256x64 weight tiles,
+// 128-byte swizzle), warp 1 issues tcgen05.mma 128x256x16 into one of two 256-column
 // TMEM accumulators, warps 2..9 drain the finished accumulator (thread = row) while the other
 // one fills.  The epilogues keep values as packed bf16 pairs wherever the reference's
 // arithmetic is bf16 (one conversion or one HMUL2/HADD2 per two elements) and keep the next
@@ -42,22 +42,31 @@ namespace {
 
 using namespace sm100;
 
-constexpr int BM = 128, BK = 64, STAGES = 4, UMMA_K = 16;
+constexpr int BM = 128, BK = 64, UMMA_K = 16;   // BM: accumulator rows of one CTA
 constexpr int BN_MAX = 256;                      // accumulator tile width: 256, or 128 for the residual GEMM on few rows
 constexpr int A_BYTES = BM * BK * 2;
-constexpr int STAGE_BYTES = A_BYTES + BN_MAX * BK * 2;   // ring slots are sized for the wide tile
-constexpr int NTHREADS = 320, EPI_THREADS = 256;
+constexpr int NTHREADS = 320, EPI_WARPS = 8;
 constexpr uint32_t TMEM_COLS = 512;
+constexpr int MAX_STAGES = 6;
+
+// CG = CTAs that share an accumulator tile.  A CTA loads its 128 rows of x and 1 / CG of the tile's weight rows;
+// the ring takes 192 KB either way (slots are sized for the wide tile).
+template <int CG> struct Ring {
+  static constexpr int STAGES = CG == 2 ? 6 : 4;
+  static constexpr int STAGE_BYTES = A_BYTES + BN_MAX / CG * BK * 2;
+};
 
 struct __align__(16) Control {
-  uint64_t full[STAGES], empty[STAGES], tfull[2], tempty[2];
+  uint64_t full[MAX_STAGES], empty[MAX_STAGES], tfull[2], tempty[2];
   uint32_t tmem_base;
   int abort_flag;
 };
 // ring | control | one 4 KB output staging buffer per epilogue warp | slack to align the base
 constexpr int WARP_STAGE_BYTES = 32 * 128;
-constexpr size_t STAGE_OFF = size_t(STAGES) * STAGE_BYTES + 256;
-constexpr size_t SMEM_BYTES = STAGE_OFF + 8 * WARP_STAGE_BYTES + 1024;
+constexpr size_t RING_BYTES = size_t(Ring<1>::STAGES) * Ring<1>::STAGE_BYTES;
+static_assert(RING_BYTES == size_t(Ring<2>::STAGES) * Ring<2>::STAGE_BYTES, "one shared-memory layout for both");
+constexpr size_t STAGE_OFF = RING_BYTES + 256;
+constexpr size_t SMEM_BYTES = STAGE_OFF + EPI_WARPS * WARP_STAGE_BYTES + 1024;
 static_assert(sizeof(Control) <= 256, "control block outgrew its slot");
 static_assert(SMEM_BYTES + 1024 <= 232448, "shared memory budget (dynamic + the static gain table)");
 
@@ -101,18 +110,26 @@ __device__ __forceinline__ void store_rows64(const WarpOut& w, int lane, const u
   __syncwarp();
 }
 
-// The reverse: 64 consecutive elements of this thread's row of a row-major bf16 matrix (`base` = the
-// warp's first row, column 0) -> 32 packed pairs in registers, read as whole lines through the
-// same staging buffer.  Rows beyond `rows` read as zero.
-__device__ __forceinline__ void load_rows64(unsigned char* stage, const __nv_bfloat16* base, int64_t ld, int rows, int lane,
-                                            uint32_t* v, int col) {
+// The reverse, in two steps: 64 columns of the warp's 32 rows of a row-major bf16 matrix (`base` = the warp's first row,
+// column 0), read as whole lines into registers - all eight loads are issued before any value is used, and long before
+// it is needed - and then through the same staging buffer to this thread's row as 32 packed pairs.  (Loaded and staged
+// one line at a time, each load waited for the shared-memory store before it: the residual epilogue took 19 us a tile
+// and bounded the kernel.)  Rows beyond `rows` read as zero.
+__device__ __forceinline__ void load_rows64(const __nv_bfloat16* base, int64_t ld, int rows, int lane, uint4* raw, int col) {
   const int sub = lane >> 3, ch = lane & 7;
 #pragma unroll
   for (int k = 0; k < 8; ++k) {
     const int r = 4 * k + sub;
-    uint4 val = make_uint4(0u, 0u, 0u, 0u);
-    if (r < rows) val = *reinterpret_cast<const uint4*>(base + int64_t(r) * ld + col + ch * 8);
-    *reinterpret_cast<uint4*>(stage + r * 128 + ((ch ^ (r & 7)) << 4)) = val;
+    raw[k] = make_uint4(0u, 0u, 0u, 0u);
+    if (r < rows) raw[k] = *reinterpret_cast<const uint4*>(base + int64_t(r) * ld + col + ch * 8);
+  }
+}
+__device__ __forceinline__ void rows64_to_row(unsigned char* stage, int lane, const uint4* raw, uint32_t* v) {
+  const int sub = lane >> 3, ch = lane & 7;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const int r = 4 * k + sub;
+    *reinterpret_cast<uint4*>(stage + r * 128 + ((ch ^ (r & 7)) << 4)) = raw[k];
   }
   __syncwarp();
 #pragma unroll
@@ -124,29 +141,30 @@ __device__ __forceinline__ void load_rows64(unsigned char* stage, const __nv_bfl
 }
 
 // ---- residual epilogue: 64 output columns of one row -------------------------------------------
-// out = resid + round_bf16(acc), a bf16 add (src/algebraic/model.py:183, 193: `x + a @ w`, both bf16);
-// returns the sum of squares of the 64 values written.
-__device__ __forceinline__ float resid_cols(const ProjParams& p, uint32_t taddr, const WarpOut& wo, const __nv_bfloat16* rbase,
-                                            int lane, int col) {
-  uint32_t res[32], out[32];
-  load_rows64(wo.stage, rbase, p.ld_resid, wo.rows, lane, res, col);
-  float ss = 0.f;
+// out = round_bf16(resid + acc) (src/algebraic/model.py:183, 193: `x + a @ w`, where the reference also rounds the
+// product on its own; one rounding is the closer of the two to the exact sum).  `res`: this row's residual values; returns the sum of squares of the 64 values written.
+__device__ __forceinline__ float resid_cols(uint32_t taddr, const WarpOut& wo, uint32_t* res, int lane, int col) {
+  float2 ss = make_float2(0.f, 0.f);
+  uint32_t r0[32], r1[32];
+  tmem_ld_32x32(taddr, r0);
+  tmem_ld_wait_for(r0);
+  tmem_ld_32x32(taddr + 32, r1);
 #pragma unroll
   for (int c = 0; c < 2; ++c) {
-    uint32_t r[32];
-    tmem_ld_32x32(taddr + c * 32, r);
-    tmem_ld_wait();
+    const uint32_t* r = c == 0 ? r0 : r1;
+    if (c == 1) tmem_ld_wait_for(r1);
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
-      const uint32_t prod = pack_bf16(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
-      const uint32_t y = as_u32(__hadd2(as_bf162(res[c * 16 + i]), as_bf162(prod)));
-      out[c * 16 + i] = y;
-      ss = fmaf(pair_lo(y), pair_lo(y), ss);
-      ss = fmaf(pair_hi(y), pair_hi(y), ss);
+      const uint32_t x = res[c * 16 + i];
+      const float2 sum = __fadd2_rn(make_float2(pair_lo(x), pair_hi(x)), make_float2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])));
+      const uint32_t y = pack_bf16(sum.x, sum.y);
+      res[c * 16 + i] = y;
+      const float2 v = make_float2(pair_lo(y), pair_hi(y));
+      ss = __ffma2_rn(v, v, ss);
     }
   }
-  store_rows64(wo, lane, out, col);
-  return ss;
+  store_rows64(wo, lane, res, col);
+  return ss.x + ss.y;
 }
 
 // tau of this row for a projection whose input is the un-normalised residual stream: the partial sums
@@ -364,32 +382,42 @@ __device__ __forceinline__ void glu_cols(const ProjParams& p, uint32_t t_gate, u
   store_rows64(wo, lane, o, col);
 }
 
-template <int EPI, int D, int BN>
+template <int EPI, int D, int BN, int CG>
 __global__ void __launch_bounds__(NTHREADS, 1)
 proj_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w, const ProjParams p) {
+  constexpr int STAGES = Ring<CG>::STAGES, STAGE_BYTES = Ring<CG>::STAGE_BYTES;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  Control* ctl = reinterpret_cast<Control*>(smem + size_t(STAGES) * STAGE_BYTES);
+  Control* ctl = reinterpret_cast<Control*>(smem + RING_BYTES);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  constexpr uint32_t IDESC = make_idesc_bf16(BM, BN, 0, 0);
+  const int rank = CG == 2 ? int(cluster_rank()) : 0;  // rank 0 issues the pair's MMAs
+  constexpr uint32_t IDESC = make_idesc_bf16(BM * CG, BN, 0, 0);
   __shared__ __align__(16) float s_gain[2 * 128];      // QKV epilogue: q gains [0,128), k gains [128,256)
   if (EPI == EPI_QKV && threadIdx.x < 2 * D) {
     const float* g = (threadIdx.x < D) ? p.q_gain : p.k_gain;
     s_gain[(threadIdx.x / D) * 128 + threadIdx.x % D] = (g != nullptr) ? g[threadIdx.x % D] : 1.0f;
   }
 
+  // full: bytes of both CTAs on the leader's barrier; empty, tfull: the leader's commits arrive in both CTAs;
+  // tempty: every epilogue warp of both CTAs on the leader's
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&ctl->full[s], 1); mbar_init(&ctl->empty[s], 1); }
-    for (int b = 0; b < 2; ++b) { mbar_init(&ctl->tfull[b], 1); mbar_init(&ctl->tempty[b], EPI_THREADS); }
+    for (int b = 0; b < 2; ++b) { mbar_init(&ctl->tfull[b], 1); mbar_init(&ctl->tempty[b], CG * EPI_WARPS); }
     ctl->abort_flag = 0;
     fence_barrier_init();
+    tma_prefetch_desc(&tm_x);
+    tma_prefetch_desc(&tm_w);
   }
   if (warp == 1) {
-    tmem_alloc(&ctl->tmem_base, TMEM_COLS);
-    tmem_relinquish();
+    if (CG == 2) {
+      tmem_alloc_pair(&ctl->tmem_base, TMEM_COLS);
+    } else {
+      tmem_alloc(&ctl->tmem_base, TMEM_COLS);
+      tmem_relinquish();
+    }
   }
   tc_fence_before();
-  __syncthreads();
+  if (CG == 2) cluster_sync_all(); else __syncthreads();
   tc_fence_after();
   // Launched as a programmatic dependent: everything above overlapped the tail of the kernel ahead in the
   // stream; from here on its results are complete.
@@ -397,23 +425,28 @@ proj_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
   const uint32_t tmem_base = ctl->tmem_base;
   const BoundedWait bw{&ctl->abort_flag, 1000000000ull};
   const int tiles_n = (p.N + BN - 1) / BN;
-  const int tiles = ((p.M + BM - 1) / BM) * tiles_n;
+  const int tiles = ((p.M + CG * BM - 1) / (CG * BM)) * tiles_n;
   const int kblocks = p.K / BK;
+  const int unit0 = blockIdx.x / CG, units = gridDim.x / CG;
 
   if (warp == 0) {
     if (lane == 0) {
-      tma_prefetch_desc(&tm_x);
-      tma_prefetch_desc(&tm_w);
       uint32_t stage = 0, phase = 0;
       bool ok = true;
-      for (int u = blockIdx.x; u < tiles && ok; u += gridDim.x) {
-        const int m = u / tiles_n, n = u % tiles_n;
+      for (int u = unit0; u < tiles && ok; u += units) {
+        const int row = (u / tiles_n * CG + rank) * BM, col = u % tiles_n * BN + rank * (BN / CG);
         for (int kb = 0; kb < kblocks; ++kb) {
           if (!bw.wait(&ctl->empty[stage], phase ^ 1u)) { ok = false; break; }
           unsigned char* dst = smem + size_t(stage) * STAGE_BYTES;
-          mbar_arrive_expect_tx(&ctl->full[stage], A_BYTES + BN * BK * 2);
-          tma_load_2d(dst, &tm_x, &ctl->full[stage], kb * BK, m * BM);
-          tma_load_2d(dst + A_BYTES, &tm_w, &ctl->full[stage], kb * BK, n * BN);
+          if (rank == 0) mbar_arrive_expect_tx(&ctl->full[stage], CG * A_BYTES + BN * BK * 2);
+          if (CG == 2) {
+            const uint32_t bar = leader_smem(&ctl->full[stage]);
+            tma_load_2d_pair(dst, &tm_x, bar, kb * BK, row);
+            tma_load_2d_pair(dst + A_BYTES, &tm_w, bar, kb * BK, col);
+          } else {
+            tma_load_2d(dst, &tm_x, &ctl->full[stage], kb * BK, row);
+            tma_load_2d(dst + A_BYTES, &tm_w, &ctl->full[stage], kb * BK, col);
+          }
           if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
       }
@@ -424,8 +457,9 @@ proj_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
     uint32_t stage = 0, phase = 0, tile_count = 0;
     const uint32_t a_lo0 = sw128_desc_lo(smem_u32(smem), 16), b_lo0 = sw128_desc_lo(smem_u32(smem) + A_BYTES, 16);
     auto wait_all = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, bw.wait(bar, parity)) != 0; };
-    bool ok = true;
-    for (int u = blockIdx.x; u < tiles && ok; u += gridDim.x, ++tile_count) {
+    auto commit = [](uint64_t* bar) { if (CG == 2) umma_commit_pair(bar); else umma_commit(bar); };
+    bool ok = rank == 0;
+    for (int u = unit0; u < tiles && ok; u += units, ++tile_count) {
       const uint32_t buf = tile_count & 1u, tphase = (tile_count >> 1) & 1u;
       if (!wait_all(&ctl->tempty[buf], tphase ^ 1u)) { ok = false; break; }
       tc_fence_after();
@@ -436,11 +470,13 @@ proj_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
         if (elect_one()) {
           const uint32_t a_lo = a_lo0 + stage * (STAGE_BYTES >> 4), b_lo = b_lo0 + stage * (STAGE_BYTES >> 4);
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k)
-            umma_f16_ss_parts(d_tmem, a_lo + k * (UMMA_K * 2 >> 4), SW128_DESC_HI, b_lo + k * (UMMA_K * 2 >> 4),
-                              SW128_DESC_HI, IDESC, (kb | k) != 0 ? 1u : 0u);
-          umma_commit(&ctl->empty[stage]);             // smem stage is free once these MMAs retire
-          if (kb == kblocks - 1) umma_commit(&ctl->tfull[buf]);   // accumulator tile complete
+          for (int k = 0; k < BK / UMMA_K; ++k) {
+            const uint32_t da = a_lo + k * (UMMA_K * 2 >> 4), db = b_lo + k * (UMMA_K * 2 >> 4);
+            if (CG == 2) umma_f16_ss_pair(d_tmem, da, SW128_DESC_HI, db, SW128_DESC_HI, IDESC, (kb | k) != 0 ? 1u : 0u);
+            else umma_f16_ss_parts(d_tmem, da, SW128_DESC_HI, db, SW128_DESC_HI, IDESC, (kb | k) != 0 ? 1u : 0u);
+          }
+          commit(&ctl->empty[stage]);                  // smem stage is free once these MMAs retire
+          if (kb == kblocks - 1) commit(&ctl->tfull[buf]);   // accumulator tile complete
         }
         __syncwarp();
         if (++stage == STAGES) { stage = 0; phase ^= 1u; }
@@ -455,8 +491,8 @@ proj_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
     uint32_t tile_count = 0;
     float best_q = 0.f, best_k = 0.f, best_v = 0.f;
     bool ok = true;
-    for (int u = blockIdx.x; u < tiles && ok; u += gridDim.x, ++tile_count) {
-      const int m = u / tiles_n, n = u % tiles_n;
+    for (int u = unit0; u < tiles && ok; u += units, ++tile_count) {
+      const int m = u / tiles_n * CG + rank, n = u % tiles_n;
       const uint32_t buf = tile_count & 1u, tphase = (tile_count >> 1) & 1u;
       const int row = m * BM + row_in_tile;
       const bool live = row < p.M;
@@ -476,12 +512,18 @@ proj_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
           ts[4 * i] = sv.x; ts[4 * i + 1] = sv.y; ts[4 * i + 2] = sv.z; ts[4 * i + 3] = sv.w;
         }
       }
+      // RESID: likewise the first 64 columns of the residual
+      const int wrow = m * BM + quarter * 32;            // first row of this warp
+      const int wrows = min(32, max(0, p.M - wrow));
+      const __nv_bfloat16* rbase = EPI == EPI_RESID ? p.resid + int64_t(wrow) * p.ld_resid : nullptr;
+      const int col0 = n * BN + half * (BN / 2);         // RESID: this thread's first column of BN / 2
+      uint4 raw[EPI == EPI_RESID ? 8 : 1];
+      if (EPI == EPI_RESID) load_rows64(rbase, p.ld_resid, col0 < p.N ? wrows : 0, lane, raw, col0);
       const float tau_row = (EPI == EPI_QKV || EPI == EPI_GLU) ? row_tau(p, row, live) : 1.0f;   // before the wait, like the table rows
       if (!bw.wait(&ctl->tfull[buf], tphase)) { ok = false; break; }
       tc_fence_after();
       const uint32_t tbuf = tmem_base + lane_sel + buf * BN;
-      const int wrow = m * BM + quarter * 32;            // first row of this warp
-      const WarpOut wo{stage, p.out + int64_t(wrow) * p.ld_out, p.ld_out, min(32, max(0, p.M - wrow))};
+      const WarpOut wo{stage, p.out + int64_t(wrow) * p.ld_out, p.ld_out, wrows};
       if (EPI == EPI_QKV) {
 #pragma unroll 1
         for (int hh = 0; hh < 128 / D; ++hh) {
@@ -502,12 +544,16 @@ proj_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
         dz_cols(p, tbuf + half * 128, wo, lane, n * BN + half * 128, a_i, inv_l, tgt);
       } else if (EPI == EPI_RESID) {
         // this thread's BN / 2 columns of its row, 64 at a time; one partial sum of squares per thread
-        const __nv_bfloat16* rbase = p.resid + int64_t(wrow) * p.ld_resid;
         float ss = 0.f;
-#pragma unroll 1
+#pragma unroll
         for (int u64 = 0; u64 < BN / 128; ++u64) {
-          const int lcol = half * (BN / 2) + u64 * 64;
-          if (n * BN + lcol < p.N) ss += resid_cols(p, tbuf + lcol, wo, rbase, lane, n * BN + lcol);
+          const int col = col0 + u64 * 64;
+          if (col < p.N) {
+            uint32_t res[32];
+            rows64_to_row(stage, lane, raw, res);
+            if (u64 + 1 < BN / 128) load_rows64(rbase, p.ld_resid, col + 64 < p.N ? wrows : 0, lane, raw, col + 64);
+            ss += resid_cols(tbuf + half * (BN / 2) + u64 * 64, wo, res, lane, col);
+          }
         }
         if (p.ss_out != nullptr && live) p.ss_out[int64_t(n * 2 + half) * p.M + row] = ss;
       } else {
@@ -516,7 +562,11 @@ proj_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
           glu_cols(p, tbuf + half * 64, tbuf + 128 + half * 64, wo, lane, fcol, tau_row);
       }
       tc_fence_before();
-      mbar_arrive(&ctl->tempty[buf]);                    // this thread is done reading the buffer
+      __syncwarp();
+      if (lane == 0) {                                   // this warp is done reading the buffer
+        if (CG == 2) mbar_arrive_cluster(leader_smem(&ctl->tempty[buf]));
+        else mbar_arrive(&ctl->tempty[buf]);
+      }
     }
     if (EPI == EPI_QKV && p.guard != nullptr) {          // one atomic per warp and statistic
       float m[3] = {warp_max(best_q), warp_max(best_k), warp_max(best_v)};
@@ -539,32 +589,51 @@ proj_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
     }
     __syncthreads();
   }
+  // a pair leaves together: until then either may still read the other's shared memory or arrive in it
+  if (CG == 2) cluster_sync_all();
   if (warp == 1) {
     __syncwarp();
     tc_fence_after();
-    tmem_dealloc(tmem_base, TMEM_COLS);
+    if (CG == 2) tmem_dealloc_pair(tmem_base, TMEM_COLS);
+    else tmem_dealloc(tmem_base, TMEM_COLS);
   }
 }
 
-template <int EPI, int D, int BN = BN_MAX>
+template <int EPI, int D, int BN, int CG>
 int launch_variant(const CUtensorMap& tm_x, const CUtensorMap& tm_w, const ProjParams& p, int grid, cudaStream_t stream) {
-  auto kern = proj_tc_kernel<EPI, D, BN>;
+  auto kern = proj_tc_kernel<EPI, D, BN, CG>;
   static PerDeviceOnce configured;
   if (int rc = configured.run([&] { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(SMEM_BYTES)); })) return rc;
-  ALG_CUDA_TRY(launch_dependent(kern, dim3(grid), dim3(NTHREADS), SMEM_BYTES, stream, tm_x, tm_w, p));
+  ALG_CUDA_TRY(launch_dependent_cluster(CG, kern, dim3(grid), dim3(NTHREADS), SMEM_BYTES, stream, tm_x, tm_w, p));
   count_launch();
   return ALG_OK;
+}
+
+template <int CG>
+int launch_cg(const CUtensorMap& tm_x, const CUtensorMap& tm_w, const ProjParams& p, int epi, int bn, int grid, cudaStream_t stream) {
+  if (epi == EPI_RESID) {
+    if constexpr (CG == 1) {
+      if (bn == 128) return launch_variant<EPI_RESID, 64, 128, 1>(tm_x, tm_w, p, grid, stream);
+    }
+    return launch_variant<EPI_RESID, 64, 256, CG>(tm_x, tm_w, p, grid, stream);
+  }
+  if (epi == EPI_GLU) return launch_variant<EPI_GLU, 64, 256, CG>(tm_x, tm_w, p, grid, stream);
+  if (epi == EPI_DZ) return launch_variant<EPI_DZ, 64, 256, CG>(tm_x, tm_w, p, grid, stream);
+  return p.D == 64 ? launch_variant<EPI_QKV, 64, 256, CG>(tm_x, tm_w, p, grid, stream)
+                   : launch_variant<EPI_QKV, 128, 256, CG>(tm_x, tm_w, p, grid, stream);
 }
 
 }  // namespace
 
 // The residual GEMM's tile is 128 x 256 unless 128 x 128 tiles spread better over the SMs (few rows: a
 // rank's share of a batch split over many GPUs).  Cost model: rounds of tiles per CTA times the time of
-// one tile, a narrow tile taking a little more than half of a wide one.
+// one tile.  A narrow tile takes a little more than half of a wide one while its rows come from L2; from HBM about
+// two thirds, its operands being 32 KB per 256 cycles of products (K = 2688, N = 1024: 8192 rows, 44 MB, 34.0 us narrow
+// and 37.8 wide; 16384 rows 94 us in 7 narrow rounds and 70 in 4 wide ones).
 int proj_resid_tile_width(int M, int N) {
   const int sms = sm_count(), mt = (M + BM - 1) / BM;
   const int wide = mt * ((N + 255) / 256), narrow = mt * ((N + 127) / 128);
-  const double cost_wide = double((wide + sms - 1) / sms), cost_narrow = 0.55 * double((narrow + sms - 1) / sms);
+  const double cost_wide = double((wide + sms - 1) / sms), cost_narrow = (M <= 8192 ? 0.55 : 0.67) * double((narrow + sms - 1) / sms);
   return cost_narrow < cost_wide ? 128 : 256;
 }
 
@@ -577,22 +646,18 @@ int launch_proj(const ProjParams& p, const void* x, const void* w, int epi, cuda
     const uint32_t box[2] = {BK, BM};
     if (int rc = make_tmap_bf16(&tm_x, x, 2, dims, strides, box, true)) return rc;
   }
-  const int bn = epi == 3 ? proj_resid_tile_width(p.M, p.N) : BN_MAX;
+  const int bn = epi == EPI_RESID ? proj_resid_tile_width(p.M, p.N) : BN_MAX;
+  const int cg = bn == BN_MAX ? pair_size((p.M + BM - 1) / BM, (p.N + bn - 1) / bn, p.K / BK) : 1;
   {
     const uint64_t dims[2] = {uint64_t(p.K), uint64_t(p.N)};
     const uint64_t strides[1] = {uint64_t(p.K)};
-    const uint32_t box[2] = {BK, uint32_t(bn)};
+    const uint32_t box[2] = {BK, uint32_t(bn / cg)};
     if (int rc = make_tmap_bf16(&tm_w, w, 2, dims, strides, box, true)) return rc;
   }
-  const int sms = sm_count();
-  const int tiles = ((p.M + BM - 1) / BM) * ((p.N + bn - 1) / bn);
-  const int grid = tiles < sms ? tiles : sms;
-  if (epi == 3) return bn == 128 ? launch_variant<EPI_RESID, 64, 128>(tm_x, tm_w, p, grid, stream)
-                                 : launch_variant<EPI_RESID, 64, 256>(tm_x, tm_w, p, grid, stream);
-  if (epi == 1) return launch_variant<EPI_GLU, 64>(tm_x, tm_w, p, grid, stream);
-  if (epi == 2) return launch_variant<EPI_DZ, 64>(tm_x, tm_w, p, grid, stream);
-  return p.D == 64 ? launch_variant<EPI_QKV, 64>(tm_x, tm_w, p, grid, stream)
-                   : launch_variant<EPI_QKV, 128>(tm_x, tm_w, p, grid, stream);
+  const int places = sm_count() / cg;
+  const int tiles = ((p.M + cg * BM - 1) / (cg * BM)) * ((p.N + bn - 1) / bn);
+  const int grid = (tiles < places ? tiles : places) * cg;
+  return cg == 2 ? launch_cg<2>(tm_x, tm_w, p, epi, bn, grid, stream) : launch_cg<1>(tm_x, tm_w, p, epi, bn, grid, stream);
 }
 
 }  // namespace alg

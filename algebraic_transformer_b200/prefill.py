@@ -130,13 +130,10 @@ class Prefill:
             raise ValueError("fused projections need head_dim 64/128, d_model % 64 == 0, d_ff % 128 == 0")
         self.fused_proj = can_fuse if fused_proj is None else bool(fused_proj)
         # `fused_norm`: the block norms as row scales inside the projections and the residual adds inside
-        # the out- and down-projection (five GEMM launches per block, no stand-alone norm).  Measured
-        # against stand-alone norms + library GEMMs with the residual in their epilogue: 3-4 % faster
-        # per step up to 4096 tokens per call (a rank's share of a batch split over several GPUs), 2-5 %
-        # slower at 16384, where the library's two-CTA 256 x 256 tiles win.  None = choose per call by the
-        # token count; the weights are laid out once for both (norm gains folded into the q|k|v and
-        # gate|up weights either way: above 4096 tokens the library takes the residual GEMMs, a pass that
-        # only reads x leaves the row statistic, and the norms still ride in the two wide projections).
+        # the out- and down-projection (five GEMM launches per block, no stand-alone norm).  None = wherever the
+        # projections are fused.  Measured against stand-alone norms + library GEMMs with the residual in
+        # their epilogue, hidden states of one call: 125M 16384 tokens 3.24 ms against 3.34, 350M 16384 tokens 10.5
+        # against 11.0, 1B 16384 tokens 29-31 against 32; 3-4 % faster up to 4096 tokens.
         if fused_norm and not self.fused_proj:
             raise ValueError("fused_norm needs the fused projections")
         self.fused_norm = fused_norm if (fused_norm is None or not self.fused_proj) else bool(fused_norm)
@@ -157,10 +154,9 @@ class Prefill:
         d, H, D, f = cfg.d_model, cfg.n_heads, cfg.head_dim, cfg.d_ff
         x = ops.rms_norm(p["embed"][tokens].contiguous(), p["embed_gain"], cfg.eps).view(B * T, d)
         attn_out = torch.empty((B, T, H, D), dtype=torch.bfloat16, device=self.device)
-        use_fused_norm = (B * T <= 4096) if self.fused_norm is None else self.fused_norm
         if self.fused_proj:
             self.guard_words.zero_()
-        if use_fused_norm:
+        if self.norm_in_weights:
             # x stays the un-normalised residual stream; `ss` carries the row statistic of the next norm
             ss = ops.row_sumsq(x)
             for layer in range(cfg.n_layers):
@@ -175,27 +171,8 @@ class Prefill:
                 ff = ops.glu_projection(x, p["w_gu_t"][layer], cfg.alu_beta, row_ss=ss, eps=cfg.eps)
                 x, ss = ops.resid_projection(ff, p["w_d_t"][layer], x, out=x)
             return ops.rms_norm(x, p["final_gain"], cfg.eps).view(B, T, d)
-        # with the gains folded into the weights the stand-alone norms run without one
-        ln1 = (lambda l: None) if self.norm_in_weights else (lambda l: p["ln1"][l])
-        ln2 = (lambda l: None) if self.norm_in_weights else (lambda l: p["ln2"][l])
-        w_o = (lambda l: p["w_o_t"][l].t()) if self.norm_in_weights else (lambda l: p["w_o"][l])
-        w_d = (lambda l: p["w_d_t"][l].t()) if self.norm_in_weights else (lambda l: p["w_d"][l])
         for layer in range(cfg.n_layers):
-            if self.norm_in_weights:
-                # library residual GEMMs, but the block norms still ride in the two wide projections: a pass
-                # that only reads x for its row statistic replaces one that reads x and writes norm(x)
-                qkv = ops.qkv_projection(x, p["w_qkv_t"][layer], H, T, self.cos_lp, self.sin_lp, p["q_gain"][layer],
-                                         p["k_gain"][layer], cfg.eps, cfg.attn_c, self.guard_words[layer],
-                                         row_ss=ops.row_sumsq(x), guard_is_zero=True).view(B, T, 3, H, D)
-                q, k, v = (qkv[:, :, i].transpose(1, 2) for i in range(3))      # (B,H,T,D) views
-                ops.flash_attention(q, k, v, p["sink"][layer], kind="asinh", n=cfg.attn_n, c=cfg.attn_c, block=T,
-                                    range_guard=True, impl=self.impl, guard_words=self.guard_words[layer],
-                                    out=attn_out.transpose(1, 2))
-                x = torch.addmm(x, attn_out.view(B * T, d), w_o(layer))
-                ff = ops.glu_projection(x, p["w_gu_t"][layer], cfg.alu_beta, row_ss=ops.row_sumsq(x), eps=cfg.eps)
-                x = torch.addmm(x, ff, w_d(layer))
-                continue
-            h = ops.rms_norm(x, ln1(layer), cfg.eps)
+            h = ops.rms_norm(x, p["ln1"][layer], cfg.eps)
             if self.fused_proj:
                 qkv = ops.qkv_projection(h, p["w_qkv_t"][layer], H, T, self.cos_lp, self.sin_lp, p["q_gain"][layer],
                                          p["k_gain"][layer], cfg.eps, cfg.attn_c, self.guard_words[layer],
@@ -204,9 +181,9 @@ class Prefill:
                 ops.flash_attention(q, k, v, p["sink"][layer], kind="asinh", n=cfg.attn_n, c=cfg.attn_c, block=T,
                                     range_guard=True, impl=self.impl, guard_words=self.guard_words[layer],
                                     out=attn_out.transpose(1, 2))
-                x = torch.addmm(x, attn_out.view(B * T, d), w_o(layer))
-                h2 = ops.rms_norm(x, ln2(layer), cfg.eps)
-                x = torch.addmm(x, ops.glu_projection(h2, p["w_gu_t"][layer], cfg.alu_beta), w_d(layer))
+                x = torch.addmm(x, attn_out.view(B * T, d), p["w_o"][layer])
+                h2 = ops.rms_norm(x, p["ln2"][layer], cfg.eps)
+                x = torch.addmm(x, ops.glu_projection(h2, p["w_gu_t"][layer], cfg.alu_beta), p["w_d"][layer])
                 continue
             qkv = torch.mm(h, p["w_qkv"][layer]).view(B, T, 3, H, D)
             q, k, v = (qkv[:, :, i].transpose(1, 2) for i in range(3))          # (B,H,T,D) views

@@ -426,7 +426,7 @@ ALG_API int alg_glu_proj_fwd(const alg_glu_proj_args* args, void* stream);
 
 /* The block's out-projection and down-projection with their residual add:
  *   out = resid + x . w^T        Replaces: `x + a @ w_o`, `x + (gate * act) @ w_d`   src/algebraic/model.py:183, 193
- * (the product rounded to bf16, then a bf16 add, as the reference's bf16 expression does), and, when
+ * (added in fp32 and rounded to bf16 once; the reference also rounds the product on its own), and, when
  * ss_out is given, per row the sum of squares of what was written, as alg_resid_proj_ss_slots(M, N)
  * partials of M floats each — what the NEXT projection needs to apply the RMS norm that follows in
  * the reference (model.py:141-143) without a pass of its own (`row_ss` of alg_qkv_proj_fwd /
