@@ -53,6 +53,15 @@ def attention(q, k, v, sink_logit: Optional[torch.Tensor] = None, *, n: int = 16
     return _Attention.apply(q, k, v, sink_logit, int(n), float(c), bool(causal), bool(range_guard))
 
 
+def _scaled(x, g, dtype):
+    # the kernel where nothing has to see the operation: not while it is recorded for a second derivative, under
+    # vmap (the cotangent is then a wrapper without storage), or for a leaf of another type
+    if torch.is_grad_enabled() or not torch._C._has_storage(g) or g.dtype != torch.float32 \
+            or dtype not in (torch.float32, torch.bfloat16):
+        return (x.float() * g).to(dtype)
+    return ops.scale_by(x, g, dtype)
+
+
 class _HeadLoss(torch.autograd.Function):
     @staticmethod
     def forward(ctx, h, embed, targets, kind, n, c):
@@ -70,7 +79,7 @@ class _HeadLoss(torch.autograd.Function):
         h, e, t, stats = ctx.saved_tensors
         dh, de = ops.fused_head_backward(h, e, t, stats, n=ctx.n, c=ctx.c, kind=ctx.kind)
         # the kernels ran with a unit cotangent; the real one is a device scalar and scales both results
-        return (dh.float() * g_obj).to(h.dtype), (de.float() * g_obj).to(ctx.embed_dtype), None, None, None, None
+        return _scaled(dh, g_obj, h.dtype), _scaled(de, g_obj, ctx.embed_dtype), None, None, None, None
 
 
 def head_loss(h, embed, targets, *, kind: str = "alg_ce", n: int = 8, c: float = 2.0):

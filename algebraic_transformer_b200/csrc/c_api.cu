@@ -683,6 +683,15 @@ int alg_head_finalize_ce(const float* lse, const float* zt, int N, float* pt, fl
   return launch_head_finalize(lse, zt, N, /*log2n=*/-1, 1.0f, 0.0f, pt, nll, obj, sums, ticket, stream);
 }
 
+int alg_scale_bf16(const void* src, const float* scale, void* dst, int dst_dtype, size_t count, void* stream) {
+  if (count == 0) return ALG_OK;
+  if (src == nullptr || scale == nullptr || dst == nullptr || (dst_dtype != ALG_BF16 && dst_dtype != ALG_F32)) {
+    set_error("scale: null pointer, or an output type other than bf16 and float32");
+    return ALG_ERR_INVALID;
+  }
+  return launch_scale_bf16(src, scale, dst, dst_dtype, count, static_cast<cudaStream_t>(stream));
+}
+
 int alg_cast_f32_to_bf16(const float* src, void* dst, size_t count, void* stream) {
   if (count != 0 && (src == nullptr || dst == nullptr)) { set_error("cast: null argument"); return ALG_ERR_INVALID; }
   if (!aligned16(src) || !aligned16(dst)) { set_error("cast: pointers must be 16-byte aligned"); return ALG_ERR_INVALID; }

@@ -59,6 +59,7 @@ int launch_rms_bwd(const RmsBwdParams& p, int dtype, cudaStream_t stream);
 int launch_prep(const PrepParams& p, int dtype, cudaStream_t stream);
 int launch_prep_batch(const PrepBatch& batch, int dtype, cudaStream_t stream);
 int launch_cast(const float* src, void* dst, size_t count, cudaStream_t stream);
+int launch_scale_bf16(const void* src, const float* scale, void* dst, int dst_dtype, size_t count, cudaStream_t stream);
 
 // ---- attention ----------------------------------------------------------------------
 struct AttnParams {

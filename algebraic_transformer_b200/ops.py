@@ -545,6 +545,19 @@ def cast_embedding(embed: torch.Tensor) -> torch.Tensor:
 
 
 @_on_tensor_device
+def scale_by(x: torch.Tensor, scale: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
+    """`(x.float() * scale).to(dtype)` for a contiguous bf16 tensor and a float32 scalar on the device, in one pass."""
+    _require_cuda(x, scale)
+    if x.dtype != torch.bfloat16 or not x.is_contiguous() or scale.dtype != torch.float32 or scale.numel() != 1:
+        raise ValueError("scale_by needs a contiguous bf16 tensor and one float32 on the device")
+    if dtype not in _DTYPES:
+        raise ValueError("scale_by writes float32 or bfloat16")
+    out = torch.empty(x.shape, dtype=dtype, device=x.device)
+    L.check(L.load().alg_scale_bf16(x.data_ptr(), scale.data_ptr(), out.data_ptr(), _DTYPES[dtype], x.numel(), _stream()))
+    return out
+
+
+@_on_tensor_device
 def head_statistic(h, e_bf16, targets, *, n: int = 16, c: float = 16.0, vocab_offset: int = 0,
                    vocab_total: Optional[int] = None, impl: str = "auto", out=None, kind: str = "alg_ce"):
     """Per-row (l, zt) of one vocabulary shard as a (2, N) fp32 tensor: row 0 the partial

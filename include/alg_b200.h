@@ -488,6 +488,9 @@ ALG_API int alg_selftest_bounded_wait(int* status, unsigned long long budget_ns,
 /* fp32 -> bf16 cast of the embedding shard (the reference casts E per call,
  * src/algebraic/kernels/fused_head.py:165; model.py:225). */
 ALG_API int alg_cast_f32_to_bf16(const float* src, void* dst, size_t count, void* stream);
+/* dst = float(src) * *scale over `count` bf16 values, rounded once to dst_dtype (ALG_BF16 or ALG_F32); `scale` is a
+ * float in device memory. */
+ALG_API int alg_scale_bf16(const void* src, const float* scale, void* dst, int dst_dtype, size_t count, void* stream);
 
 #ifdef __cplusplus
 }

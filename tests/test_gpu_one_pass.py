@@ -1,0 +1,43 @@
+"""Passes that were joined or taken out: the head gradient's scale, the fp32 layer's preparation, the copy of an output
+gradient in another layout."""
+
+import pytest
+import torch
+
+import algebraic_transformer_b200 as A
+from algebraic_transformer_b200 import autograd as G
+from algebraic_transformer_b200 import ops
+from oracle import algebraic_ref as R
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def rel_l2(a, b):
+    a, b = a.detach().double().cpu(), b.detach().double().cpu()
+    return float((a - b).norm() / b.norm().clamp_min(1e-30))
+
+
+def randn(shape, seed, dtype=torch.float32, scale=1.0):
+    return (torch.randn(shape, generator=torch.Generator().manual_seed(seed)) * scale).to(dtype)
+
+
+@pytest.mark.parametrize("n,offset", [(0, 0), (1, 0), (7, 0), (4099, 0), (4099, 1)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_scale_by(n, offset, dtype):
+    x, s = randn((n + offset,), 61, torch.bfloat16).to(DEV)[offset:], torch.tensor(1.7, device=DEV)
+    assert torch.equal(ops.scale_by(x, s, dtype), (x.float() * s).to(dtype))
+
+
+@pytest.mark.parametrize("embed_dtype", [torch.float32, torch.bfloat16, torch.float16])
+def test_head_loss_scales_its_gradients(embed_dtype):
+    h, e = randn((65, 64), 62, torch.bfloat16).to(DEV).requires_grad_(True), randn((72, 64), 63, embed_dtype).to(DEV).requires_grad_(True)
+    t = torch.arange(65, device=DEV)
+    obj, _ = G.head_loss(h, e, t)
+    one = torch.autograd.grad(obj, (h, e), retain_graph=True)
+    two = torch.autograd.grad(obj * 3, (h, e), retain_graph=True)
+    many = torch.autograd.grad(obj, (h, e), torch.tensor([1.0, 3.0], device=DEV), retain_graph=True, is_grads_batched=True)
+    slope = torch.autograd.grad(obj * 3, (h, e), create_graph=True)
+    for a, b, c, s in zip(one, two, many, slope):
+        assert a.dtype == b.dtype and rel_l2(b, 3 * a.float()) < 5e-3      # a bf16 rounding
+        assert torch.equal(c[0], a) and torch.equal(c[1], b) and torch.equal(s, b)
