@@ -1330,8 +1330,9 @@ bool attn_tcgen05_f32_supports(const AttnParams& p, int dtype) {
 
 // p describes the fp32 problem (q, k, v, o fp32 with their strides); `split` holds three buffers of
 // attn_tcgen05_f32_split_bytes each.  Unshifted form only (under a guard the kernel leaves when the
-// guard calls for the shift, like the bf16 one).
-int launch_attn_tcgen05_f32(const AttnParams& p, void* split, cudaStream_t stream) {
+// guard calls for the shift, like the bf16 one).  `is_split`: the copies are there already (the pass that took the
+// guard's maxima left them).
+int launch_attn_tcgen05_f32(const AttnParams& p, void* split, bool is_split, cudaStream_t stream) {
   const size_t each = attn_tcgen05_f32_split_bytes(p.B, p.H, p.Tq);
   unsigned char* base = static_cast<unsigned char*>(split);
   SplitBatch batch{};
@@ -1339,11 +1340,13 @@ int launch_attn_tcgen05_f32(const AttnParams& p, void* split, cudaStream_t strea
   batch.t[0] = {static_cast<const float*>(p.q), reinterpret_cast<__nv_bfloat16*>(base), p.qs, p.Tq};
   batch.t[1] = {static_cast<const float*>(p.k), reinterpret_cast<__nv_bfloat16*>(base + each), p.ks, p.Tk};
   batch.t[2] = {static_cast<const float*>(p.v), reinterpret_cast<__nv_bfloat16*>(base + 2 * each), p.vs, p.Tk};
-  const int64_t vecs = int64_t(p.B) * p.H * p.Tq * 16;
-  int64_t blocks = (vecs + 255) / 256;
-  if (blocks > int64_t(sm_count()) * 8) blocks = int64_t(sm_count()) * 8;
-  ALG_CUDA_TRY(launch_dependent(split_f32_kernel, dim3(unsigned(blocks), 3), dim3(256), 0, stream, batch));
-  count_launch();
+  if (!is_split) {
+    const int64_t vecs = int64_t(p.B) * p.H * p.Tq * 16;
+    int64_t blocks = (vecs + 255) / 256;
+    if (blocks > int64_t(sm_count()) * 8) blocks = int64_t(sm_count()) * 8;
+    ALG_CUDA_TRY(launch_dependent(split_f32_kernel, dim3(unsigned(blocks), 3), dim3(256), 0, stream, batch));
+    count_launch();
+  }
   AttnParams ps = p;
   ps.q = batch.t[0].y; ps.k = batch.t[1].y; ps.v = batch.t[2].y;
   const Strides3 dense = {int64_t(p.H) * p.Tq * 128, int64_t(p.Tq) * 128, 128};

@@ -274,6 +274,11 @@ int alg_attn_fwd(const alg_attn_args* a, void* stream_) {
     p.tc_shift = 1;                                     // move in as the first kernel's leave and wait there for its records
     return launch_attn_tcgen05(p, stream);
   }
+  // fp32 rows of head_dim 64: the same tcgen05 kernel on bf16 hi | lo copies, when the caller's workspace has
+  // room for them; the max-shifted form (explicit, or a failed guard) stays on the mma.sync kernel
+  const size_t split_off = align256(need), split_each = align256(attn_tcgen05_f32_split_bytes(a->B, a->H, a->Tq));
+  const bool f32_tc = attn_tcgen05_f32_supports(p, a->dtype) && a->variant != ALG_VARIANT_SHIFT && !(a->score_clamp > 0.0f) &&
+                      a->impl != ALG_IMPL_MMA && ws != nullptr && aligned16(ws) && a->workspace_bytes >= split_off + 3 * split_each;
   if (guarded && !guard_given) ALG_CUDA_TRY(cudaMemsetAsync(guard, 0, sizeof(GuardWords), stream));
   if (prologue || (guarded && !guard_given)) {
     const size_t es = elem_size(a->dtype);
@@ -295,15 +300,13 @@ int alg_attn_fwd(const alg_attn_args* a, void* stream_) {
     pp.stat_scale = 1.0f; pp.stat_out = &guard->k2;
     batch.t[batch.count++] = pp;
     if (guarded) {                                      // v: max |v| only
-      if (prologue) {                                   // q,k are normalised in their own launch
-        if (int rc = launch_prep_batch(batch, a->dtype, stream)) return rc;
-        batch.count = 0;
-      }
       pp.x = a->v; pp.xs = p.vs; pp.y = nullptr; pp.gain = nullptr; pp.cos = nullptr; pp.sin = nullptr;
       pp.normalise = 0; pp.stat_mode = 2; pp.stat_out = &guard->vmax;
       batch.t[batch.count++] = pp;
     }
-    if (int rc = launch_prep_batch(batch, a->dtype, stream)) return rc;  // statistics-only tensors share a launch
+    // the pass over q, k and v leaves the hi | lo copies the fp32 kernel reads (a pass of its own read all three again)
+    for (int i = 0; f32_tc && guarded && i < 3; ++i) batch.t[i].split = ws + split_off + size_t(i) * split_each;
+    if (int rc = launch_prep_batch(batch, a->dtype, stream)) return rc;
     if (prologue) {
       p.q = qn; p.k = kn;
       p.qs = strides_or_dense(kDense, a->H, a->Tq, a->D);
@@ -311,14 +314,9 @@ int alg_attn_fwd(const alg_attn_args* a, void* stream_) {
     }
   }
 
-  // fp32 rows of head_dim 64: the same tcgen05 kernel on bf16 hi | lo copies, when the caller's workspace has
-  // room for them; the max-shifted form (explicit, or a failed guard) stays on the mma.sync kernel
-  const size_t split_off = align256(need), split_each = align256(attn_tcgen05_f32_split_bytes(a->B, a->H, a->Tq));
-  const bool f32_tc = attn_tcgen05_f32_supports(p, a->dtype) && a->variant != ALG_VARIANT_SHIFT && !(a->score_clamp > 0.0f) &&
-                      a->impl != ALG_IMPL_MMA && ws != nullptr && aligned16(ws) && a->workspace_bytes >= split_off + 3 * split_each;
   if (f32_tc) {
     p.run_if = guarded ? 1 : 0;
-    if (int rc = launch_attn_tcgen05_f32(p, ws + split_off, stream)) return rc;
+    if (int rc = launch_attn_tcgen05_f32(p, ws + split_off, guarded && !guard_given, stream)) return rc;
     if (!guarded) return ALG_OK;
     p.run_if = 2;                                       // the max-shifted form runs only if the guard failed
     return launch_attn_mma(p, a->dtype, stream);

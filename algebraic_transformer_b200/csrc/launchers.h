@@ -37,6 +37,7 @@ struct PrepParams {
   int stat_mode;           // 0 none, 1 max squared row norm of round(x*stat_scale), 2 max |x|
   float stat_scale;
   unsigned* stat_out;
+  void* split;             // fp32 rows of head_dim 64: (B, H, T, 128) bf16 hi | lo copy of the result, or nullptr
 };
 struct PrepBatch {         // up to three tensors (q, k, v) of one dtype / head_dim in one launch
   PrepParams t[3];
@@ -102,7 +103,7 @@ int launch_attn_tcgen05(const AttnParams& p, cudaStream_t stream);
 // buffers of attn_tcgen05_f32_split_bytes each, at `split`); unshifted form, fp32 output
 bool attn_tcgen05_f32_supports(const AttnParams& p, int dtype);
 size_t attn_tcgen05_f32_split_bytes(int B, int H, int T);
-int launch_attn_tcgen05_f32(const AttnParams& p, void* split, cudaStream_t stream);
+int launch_attn_tcgen05_f32(const AttnParams& p, void* split, bool is_split, cudaStream_t stream);
 
 // Shared by both attention kernels: does this launch use the max-shifted form?  Called by all 32
 // lanes of one warp; every lane gets the answer.

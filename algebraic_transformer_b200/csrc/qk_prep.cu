@@ -53,8 +53,9 @@ template <> struct Vec16<__nv_bfloat16> {
 
 // MODE 0: statistics only (guard maxima of ready-made q / k / v); 1: normalise (+ gain);
 // 2: normalise + rotate.  Modes 1 and 2 can also accumulate a statistic in the same pass.
+// fp32 rows of head_dim 64 can leave their bf16 hi | lo copy (attn_sm100.cu) as well: `split`.
 template <typename T, int D, int MODE>
-__global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) qk_prep_kernel(const PrepBatch batch) {
+__device__ __forceinline__ void prep_body(const PrepParams& p) {
   using V = Vec16<T>;
   constexpr int VEC = V::N;
   constexpr int LPR = D / VEC;         // lanes per row
@@ -64,7 +65,6 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) qk_prep_kernel(const P
   // per SM in flight, which is what 6.5 TB/s needs at the loaded memory latency (with four the
   // normalising pass stopped at 5.0 TB/s; with eight it reaches 5.4).
   constexpr int HEADS_PER_STEP = 8;
-  const PrepParams& p = batch.t[blockIdx.y];
   const int lane = threadIdx.x & 31;
   const int lir = lane % LPR;          // lane in row
   const int sub = lane / LPR;
@@ -181,6 +181,16 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) qk_prep_kernel(const P
           }
         }
         if (MODE >= 1 && !(MODE == 2 && sizeof(T) == 2) && dst0 != nullptr && on) V::store(dst0 + int64_t(h) * p.ys.h, v);
+        if constexpr (sizeof(T) == 4 && D == 64) {
+          if (p.split != nullptr && on) {
+            const uint32_t h0 = pack_bf16(v[0], v[1]), h1 = pack_bf16(v[2], v[3]);
+            const uint32_t l0 = pack_bf16(v[0] - __uint_as_float(h0 << 16), v[1] - __uint_as_float(h0 & 0xffff0000u));
+            const uint32_t l1 = pack_bf16(v[2] - __uint_as_float(h1 << 16), v[3] - __uint_as_float(h1 & 0xffff0000u));
+            __nv_bfloat16* out = static_cast<__nv_bfloat16*>(p.split) + ((b * p.H + h) * p.T + t) * 128 + lir * VEC;
+            *reinterpret_cast<uint2*>(out) = make_uint2(h0, h1);
+            *reinterpret_cast<uint2*>(out + 64) = make_uint2(l0, l1);
+          }
+        }
         if (p.stat_mode == 1) {          // squared row norm of the re-rounded scaled row
           float ss = 0.0f;
 #pragma unroll
@@ -215,13 +225,21 @@ __global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) qk_prep_kernel(const P
   }
 }
 
+// Tensor blockIdx.y of the batch; a third tensor (v) of a normalising batch is read for its statistic only.
+template <typename T, int D, int MODE>
+__global__ void __launch_bounds__(256, MODE == 0 ? 4 : 3) qk_prep_kernel(const PrepBatch batch) {
+  const PrepParams& p = batch.t[blockIdx.y];
+  if (MODE != 0 && blockIdx.y == 2) prep_body<T, D, 0>(p);
+  else prep_body<T, D, MODE>(p);
+}
+
 template <typename T, int D>
 static int launch_t(const PrepBatch& batch, cudaStream_t stream) {
-  // every tensor of a batch runs the same mode (the callers group them that way)
+  // the first two tensors of a batch run the same mode, the third (v) is statistics only
   const int mode = !batch.t[0].normalise ? 0 : (batch.t[0].cos != nullptr ? 2 : 1);
   for (int i = 1; i < batch.count; ++i) {
     const int m = !batch.t[i].normalise ? 0 : (batch.t[i].cos != nullptr ? 2 : 1);
-    if (m != mode) { set_error("internal: mixed modes in one prep batch"); return ALG_ERR_INVALID; }
+    if (m != (i == 2 ? 0 : mode)) { set_error("internal: mixed modes in one prep batch"); return ALG_ERR_INVALID; }
   }
   constexpr int LPR = D * int(sizeof(T)) / 16;
   constexpr int RPW = 32 / LPR;

@@ -41,3 +41,21 @@ def test_head_loss_scales_its_gradients(embed_dtype):
     for a, b, c, s in zip(one, two, many, slope):
         assert a.dtype == b.dtype and rel_l2(b, 3 * a.float()) < 5e-3      # a bf16 rounding
         assert torch.equal(c[0], a) and torch.equal(c[1], b) and torch.equal(s, b)
+
+
+# in range (tcgen05 on the hi | lo copies) and out of range (the max-shifted form reads the fp32 rows)
+@pytest.mark.parametrize("vscale", [1.0, 1e9])
+@pytest.mark.parametrize("B,H,T", [(1, 1, 1), (2, 9, 130), (1, 3, 515)])
+def test_fp32_layer_preparation(B, H, T, vscale):
+    q, k, v = (randn((B, T, H, 64), 71 + i).transpose(1, 2) for i in range(3))
+    v = v * vscale
+    gain, sink = 0.5 + torch.rand(64, generator=torch.Generator().manual_seed(74)), randn((H,), 75, scale=0.5)
+    cos, sin = R.cayley_table_geometric(64, T)
+    want = R.asinh_attention(R.apply_rotary(R.rms_norm(q, gain), cos, sin), R.apply_rotary(R.rms_norm(k, gain), cos, sin), v,
+                             n=16, c=8.0, sink_logit=sink)
+    q, k, v, gain, sink, cos, sin = (t.to(DEV) for t in (q, k, v, gain, sink, cos, sin))
+    got = A.flash_attention(q, k, v, sink, kind="asinh", n=16, c=8.0, block=T, range_guard=True, q_gain=gain, k_gain=gain,
+                            cos=cos, sin=sin)
+    assert rel_l2(got, want) < 1e-4                                # 16 mantissa bits of weights and values
+    q, k = (A.qk_rms_norm(x, gain, cos=cos, sin=sin) for x in (q, k))
+    assert torch.equal(got, A.flash_attention(q, k, v, sink, kind="asinh", n=16, c=8.0, block=T, range_guard=True))
