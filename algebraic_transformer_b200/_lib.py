@@ -122,6 +122,7 @@ SYMBOLS = {
     "alg_attn_fwd": (C.c_int, [C.POINTER(AttnArgs), C.c_void_p]),
     "alg_attn_bwd_workspace_bytes": (C.c_size_t, [C.POINTER(AttnBwdArgs)]),
     "alg_attn_bwd": (C.c_int, [C.POINTER(AttnBwdArgs), C.c_void_p]),
+    "alg_attn_bwd_strided": (C.c_int, [C.POINTER(AttnBwdArgs), I64x3, C.c_void_p]),
     "alg_head_bwd_dz": (C.c_int, [C.POINTER(HeadBwdArgs), C.c_void_p]),
     "alg_decode_workspace_bytes": (C.c_size_t, [C.POINTER(DecodeArgs)]),
     "alg_attn_decode": (C.c_int, [C.POINTER(DecodeArgs), C.c_void_p]),

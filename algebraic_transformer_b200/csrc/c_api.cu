@@ -451,7 +451,9 @@ size_t alg_attn_bwd_workspace_bytes(const alg_attn_bwd_args* a) {
   return size_t(a->B) * a->H * a->Tq * sizeof(float);
 }
 
-int alg_attn_bwd(const alg_attn_bwd_args* a, void* stream_) {
+int alg_attn_bwd(const alg_attn_bwd_args* a, void* stream) { return alg_attn_bwd_strided(a, nullptr, stream); }
+
+int alg_attn_bwd_strided(const alg_attn_bwd_args* a, const int64_t* do_stride, void* stream_) {
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   if (a == nullptr || a->q == nullptr || a->k == nullptr || a->v == nullptr || a->o == nullptr || a->d_o == nullptr ||
       a->stat == nullptr || a->stat_kind == nullptr || a->dq == nullptr || a->dk == nullptr || a->dv == nullptr) {
@@ -488,9 +490,9 @@ int alg_attn_bwd(const alg_attn_bwd_args* a, void* stream_) {
   p.ks = strides_or_dense(a->k_stride, a->H, a->Tk, a->D);
   p.vs = strides_or_dense(a->v_stride, a->H, a->Tk, a->D);
   p.os = strides_or_dense(a->o_stride, a->H, a->Tq, a->D);
-  p.gs = p.os;
+  p.gs = do_stride != nullptr ? Strides3{do_stride[0], do_stride[1], do_stride[2]} : p.os;
   if (!strides_ok(p.qs, ALG_BF16) || !strides_ok(p.ks, ALG_BF16) || !strides_ok(p.vs, ALG_BF16) || !strides_ok(p.os, ALG_BF16) ||
-      !aligned16(a->q) || !aligned16(a->k) || !aligned16(a->v) || !aligned16(a->o) || !aligned16(a->d_o) ||
+      !strides_ok(p.gs, ALG_BF16) || !aligned16(a->q) || !aligned16(a->k) || !aligned16(a->v) || !aligned16(a->o) || !aligned16(a->d_o) ||
       !aligned16(a->dq) || !aligned16(a->dk) || !aligned16(a->dv)) {
     set_error("attention backward: rows must start on 16-byte boundaries");
     return ALG_ERR_INVALID;

@@ -46,10 +46,21 @@ int make_tmap_bf16(CUtensorMap* out, const void* base, int rank, const uint64_t*
     set_error("TMA needs a 16-byte aligned base address");
     return ALG_ERR_INVALID;
   }
-  CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, cuuint32_t(rank), const_cast<void*>(base), gdim, gstride,
-                   bdim, estride, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                   swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
-                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  auto encode = [&] {
+    return enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, cuuint32_t(rank), const_cast<void*>(base), gdim, gstride,
+               bdim, estride, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  };
+  CUresult r = encode();
+  if (r == CUDA_ERROR_INVALID_CONTEXT) {
+    // a thread whose first CUDA work this is (an autograd engine's) has a device but no context bound yet: a
+    // driver call does not bind it, the runtime's selection of the current device does
+    int dev = 0;
+    ALG_CUDA_TRY(cudaGetDevice(&dev));
+    ALG_CUDA_TRY(cudaSetDevice(dev));
+    r = encode();
+  }
   if (r != CUDA_SUCCESS) {
     set_error("cuTensorMapEncodeTiled failed with CUresult %d", int(r));
     return ALG_ERR_CUDA;

@@ -472,7 +472,10 @@ def flash_attention_backward(q, k, v, o, d_o, stat, stat_kind, sink_logit=None, 
         raise ValueError("stat must be the contiguous float32 (B, H, Tq) statistic of the forward")
     if n < 2 or n & (n - 1):
         raise ValueError("asinh kernel needs n to be a power of two")
-    if d_o.stride() != o.stride():
+    # the gradient is read in the layout it comes in where its rows are 16-byte aligned and apart; any other (an expanded
+    # gradient, an odd view) is copied into o's layout first
+    gb, gh, gt, gd = d_o.stride()
+    if d_o.stride() != o.stride() and (gd != 1 or min(gb, gh, gt) <= 0 or (gb | gh | gt) % 8 or gt < D or d_o.data_ptr() % 16):
         d_o = torch.empty_strided(o.shape, o.stride(), dtype=o.dtype, device=o.device).copy_(d_o)
     sink = None
     if sink_logit is not None:
@@ -490,7 +493,7 @@ def flash_attention_backward(q, k, v, o, d_o, stat, stat_kind, sink_logit=None, 
     lib = L.load()
     ws = _workspace(q.device, lib.alg_attn_bwd_workspace_bytes(a), "attn_bwd")
     a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
-    L.check(lib.alg_attn_bwd(a, _stream()))
+    L.check(lib.alg_attn_bwd_strided(a, _strides3(d_o), _stream()))
     return dq, dk, dv, dsink
 
 

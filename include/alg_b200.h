@@ -218,6 +218,9 @@ typedef struct {
 } alg_attn_bwd_args;
 ALG_API size_t alg_attn_bwd_workspace_bytes(const alg_attn_bwd_args* args);
 ALG_API int alg_attn_bwd(const alg_attn_bwd_args* args, void* stream);
+/* The same with d_o in a layout of its own: element strides of (B, H, Tq), D contiguous, as a projection that runs on
+ * (B, Tq, H, D) rows hands its input gradient back, without a copy into o's layout.  NULL: o's strides. */
+ALG_API int alg_attn_bwd_strided(const alg_attn_bwd_args* args, const int64_t* do_stride, void* stream);
 
 /* ------------------------------------------------------------------------------------
  * Single-query decode against a KV cache (Tq = 1, every key visible), split over keys.

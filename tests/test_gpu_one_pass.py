@@ -59,3 +59,38 @@ def test_fp32_layer_preparation(B, H, T, vscale):
     assert rel_l2(got, want) < 1e-4                                # 16 mantissa bits of weights and values
     q, k = (A.qk_rms_norm(x, gain, cos=cos, sin=sin) for x in (q, k))
     assert torch.equal(got, A.flash_attention(q, k, v, sink, kind="asinh", n=16, c=8.0, block=T, range_guard=True))
+
+
+# dense, (B, T, H, D) rows, rows apart by more than D, misaligned rows, an expanded gradient; both kernel families
+@pytest.mark.parametrize("layout", ["dense", "bthd", "wide", "odd", "expanded"])
+@pytest.mark.parametrize("impl", ["auto", "mma"])
+def test_output_gradient_layouts(layout, impl):
+    B, H, T, D = 2, 3, 130, 64
+    q, k, v = (randn((B, H, T, D), 81 + i, torch.bfloat16).to(DEV) for i in range(3))
+    sink, g = randn((H,), 84, scale=0.3).to(DEV), randn((B, T, H, D), 85, torch.bfloat16).to(DEV)
+    o, stat, which = A.flash_attention(q, k, v, sink, kind="asinh", n=16, c=8.0, block=T, range_guard=True, return_stat=True)
+    if layout == "bthd":
+        g = g.transpose(1, 2)
+    elif layout in ("wide", "odd"):
+        g = torch.zeros((B, H, T, D + (8 if layout == "wide" else 2)), dtype=torch.bfloat16, device=DEV)[..., :D].copy_(g.transpose(1, 2))
+    elif layout == "expanded":
+        g = g[:, :1, :1, :1].expand(B, H, T, D)
+    else:
+        g = g.transpose(1, 2).contiguous()
+    got = ops.flash_attention_backward(q, k, v, o, g, stat, which, sink, impl=impl)
+    want = ops.flash_attention_backward(q, k, v, o, g.contiguous(), stat, which, sink, impl=impl)
+    for a, b in zip(got[:3], want[:3]):
+        assert torch.equal(a, b)
+    assert rel_l2(got[3], want[3]) < 1e-5                          # the sink's gradient adds its blocks in any order
+
+
+def test_backward_in_a_thread_without_a_context():
+    """The first CUDA work of a thread may be the backward call: nothing before it has bound a context there."""
+    import threading
+    B, H, T, D = 1, 2, 64, 64
+    q, k, v = (randn((B, H, T, D), 91 + i, torch.bfloat16).to(DEV) for i in range(3))
+    o, stat, which = A.flash_attention(q, k, v, None, kind="asinh", n=16, c=8.0, block=T, range_guard=True, return_stat=True)
+    want, got = ops.flash_attention_backward(q, k, v, o, o, stat, which), []
+    t = threading.Thread(target=lambda: got.extend(ops.flash_attention_backward(q, k, v, o, o, stat, which)[:3]))
+    t.start(), t.join()
+    assert len(got) == 3 and all(torch.equal(a, b) for a, b in zip(got, want))
