@@ -83,6 +83,14 @@ class ResidProjArgs(C.Structure):
                 ("ld_resid", C.c_int64), ("ld_out", C.c_int64), ("status", C.c_void_p)]
 
 
+class PrefillBlocksArgs(C.Structure):
+    _fields_ = [(name, C.c_void_p) for name in ("x", "out", "w_qkv", "w_o", "w_gu", "w_d", "q_gain", "k_gain", "sink",
+                                                "final_gain", "cos", "sin", "guard")] + \
+               [(name, C.c_int) for name in ("L", "B", "T", "H", "D", "d", "f", "attn_n")] + \
+               [("attn_c", C.c_float), ("eps", C.c_float), ("alu_beta", C.c_float), ("impl", C.c_int),
+                ("workspace", C.c_void_p), ("workspace_bytes", C.c_size_t), ("status", C.c_void_p)]
+
+
 class DecodeArgs(C.Structure):
     _fields_ = [("q", C.c_void_p), ("k", C.c_void_p), ("v", C.c_void_p), ("o", C.c_void_p),
                 ("sink", C.c_void_p), ("B", C.c_int), ("H", C.c_int), ("Tk", C.c_int), ("D", C.c_int),
@@ -136,6 +144,8 @@ SYMBOLS = {
                                     C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_size_t, C.c_void_p]),
     "alg_head_finalize_ce": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p,
                                        C.c_void_p, C.c_size_t, C.c_void_p]),
+    "alg_prefill_blocks_workspace_bytes": (C.c_size_t, [C.POINTER(PrefillBlocksArgs)]),
+    "alg_prefill_blocks": (C.c_int, [C.POINTER(PrefillBlocksArgs), C.c_void_p]),
     "alg_cast_f32_to_bf16": (C.c_int, [C.c_void_p, C.c_void_p, C.c_size_t, C.c_void_p]),
     "alg_scale_bf16": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_size_t, C.c_void_p]),
     "alg_qkv_proj_fwd": (C.c_int, [C.POINTER(QkvProjArgs), C.c_void_p]),

@@ -24,7 +24,9 @@ _workspaces = {}
 
 
 def _stream():
-    return torch.cuda.current_stream().cuda_stream
+    """The current device's current stream as the pointer the C side takes (the raw query: `torch.cuda.current_stream()`
+    builds a Stream object, 3 us a call)."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _ptr(t: Optional[torch.Tensor]):
@@ -56,13 +58,15 @@ def _on_tensor_device(fn):
     @functools.wraps(fn)
     def call(*args, **kwargs):
         dev = None
-        for a in list(args) + list(kwargs.values()):
-            if isinstance(a, torch.Tensor) and a.device.type == "cuda":
-                if dev is None:
-                    dev = a.device
-                elif a.device != dev:
-                    raise ValueError(f"{fn.__name__}: tensors on different devices ({dev} and {a.device})")
-        if dev is None or dev.index == torch.cuda.current_device():
+        for a in (*args, *kwargs.values()):
+            if isinstance(a, torch.Tensor):
+                place = a.device
+                if place.type == "cuda":
+                    if dev is None:
+                        dev = place
+                    elif place != dev:
+                        raise ValueError(f"{fn.__name__}: tensors on different devices ({dev} and {place})")
+        if dev is None or dev.index == torch._C._cuda_getDevice():
             return fn(*args, **kwargs)
         with torch.cuda.device(dev):
             return fn(*args, **kwargs)
@@ -72,7 +76,16 @@ def _on_tensor_device(fn):
 def _strides3(t: torch.Tensor):
     if t.stride(-1) != 1:
         raise ValueError("the last (head_dim) axis must be contiguous")
-    return L.I64x3(t.stride(0), t.stride(1), t.stride(2))
+    b, h, r, _ = t.stride()
+    return L.I64x3(b, h, r)
+
+
+def _sink_vector(sink_logit, H: int, device):
+    """The sink logits as a contiguous float32 vector on `device`; one logit serves every head."""
+    s = sink_logit
+    if not (isinstance(s, torch.Tensor) and s.dtype == torch.float32 and s.ndim == 1 and s.device == device):
+        s = torch.as_tensor(s, dtype=torch.float32, device=device).reshape(-1)
+    return s.expand(H).contiguous() if s.numel() == 1 else s.contiguous()
 
 
 def _root(value: float, n: int) -> float:
@@ -346,6 +359,43 @@ def row_sumsq(x: torch.Tensor) -> torch.Tensor:
     return ss
 
 
+@_on_tensor_device
+def prefill_blocks(x, w_qkv, w_o, w_gu, w_d, q_gain, k_gain, sink, final_gain, cos, sin, guard_words, *, batch: int,
+                   n_heads: int, eps: float = 1e-5, alu_beta: float = 0.5, attn_n: int = 16, attn_c: float = 8.0,
+                   impl: str = "auto") -> torch.Tensor:
+    """Every block of a prefill and the final norm in one call (src/algebraic/model.py:162-208): per block the launches of
+    `qkv_projection`, `flash_attention`, `resid_projection`, `glu_projection`, `resid_projection`, with the norms as row
+    scales, issued natively.  x: (batch * T, d) bf16, the normalised embedding; it is overwritten with the last
+    block's output.  Weights are stacked over the blocks, (L, ...) contiguous bf16, in the layouts of those operators,
+    gains and sinks float32; `guard_words`: (L, 4) int32, zeroed by the caller.  Returns (batch * T, d) bf16."""
+    _require_cuda(x, w_qkv, w_o, w_gu, w_d, q_gain, k_gain, sink, final_gain, cos, sin, guard_words)
+    layers, d = w_qkv.shape[0], x.shape[1]
+    D, f, T = d // n_heads, w_gu.shape[1] // 2, x.shape[0] // batch if batch else 1
+    for name, t, shape in (("x", x, (batch * T, d)), ("w_qkv", w_qkv, (layers, 3 * d, d)), ("w_o", w_o, (layers, d, d)),
+                           ("w_gu", w_gu, (layers, 2 * f, d)), ("w_d", w_d, (layers, d, f))):
+        if t.dtype != torch.bfloat16 or t.shape != shape or not t.is_contiguous():
+            raise ValueError(f"{name} must be contiguous bf16 of shape {shape}")
+    for name, t, shape in (("q_gain", q_gain, (layers, D)), ("k_gain", k_gain, (layers, D)), ("sink", sink, (layers, n_heads)),
+                           ("final_gain", final_gain, (d,))):
+        if t.dtype != torch.float32 or t.shape != shape or not t.is_contiguous():
+            raise ValueError(f"{name} must be contiguous float32 of shape {shape}")
+    for t in (cos, sin):
+        if t.dtype != torch.bfloat16 or not t.is_contiguous() or t.shape[1] != D // 2 or t.shape[0] < T:
+            raise ValueError("rotation tables must be contiguous bf16 (>= seq_len, D/2)")
+    if guard_words.dtype != torch.int32 or guard_words.shape != (layers, 4) or not guard_words.is_contiguous():
+        raise ValueError("guard_words must be contiguous int32 (L, 4)")
+    out = torch.empty_like(x)
+    a = L.PrefillBlocksArgs(x.data_ptr(), out.data_ptr(), w_qkv.data_ptr(), w_o.data_ptr(), w_gu.data_ptr(), w_d.data_ptr(),
+                            q_gain.data_ptr(), k_gain.data_ptr(), sink.data_ptr(), final_gain.data_ptr(), cos.data_ptr(),
+                            sin.data_ptr(), guard_words.data_ptr(), layers, batch, T, n_heads, D, d, f, attn_n, attn_c, eps,
+                            alu_beta, L.IMPL[impl])
+    lib = L.load()
+    ws = torch.empty(lib.alg_prefill_blocks_workspace_bytes(a), dtype=torch.uint8, device=x.device)
+    a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
+    L.check(lib.alg_prefill_blocks(a, _stream()))
+    return out
+
+
 # ------------------------------------------------------------------------ attention
 
 def flash_clamp(seq_len: int, n: int) -> float:
@@ -420,8 +470,7 @@ def flash_attention(q, k, v, sink_logit=None, *, kind: str = "softmax", n: int =
 
     sink = None
     if sink_logit is not None:
-        s = torch.as_tensor(sink_logit, dtype=torch.float32, device=q.device).reshape(-1)
-        sink = s.expand(H).contiguous() if s.numel() == 1 else s.contiguous()
+        sink = _sink_vector(sink_logit, H, q.device)
         if sink.numel() != H:
             raise ValueError("sink_logit must broadcast to (H,)")
     for t in (q_gain, k_gain):
@@ -431,9 +480,9 @@ def flash_attention(q, k, v, sink_logit=None, *, kind: str = "softmax", n: int =
         cos, sin = cos.contiguous().float(), sin.contiguous().float()
     o = torch.empty((B, H, T, D), dtype=q.dtype, device=q.device) if out is None else out
     stat = torch.empty((B, H, T), dtype=torch.float32, device=q.device) if return_stat else None
-    stat_kind = torch.zeros(1, dtype=torch.int32, device=q.device) if return_stat else None
     if q.numel() == 0:
-        return (o, stat, stat_kind) if return_stat else o
+        return (o, stat, torch.zeros(1, dtype=torch.int32, device=q.device)) if return_stat else o
+    stat_kind = torch.empty(1, dtype=torch.int32, device=q.device) if return_stat else None    # whichever kernel runs writes it
     a = L.AttnArgs(q=q.data_ptr(), k=k.data_ptr(), v=v.data_ptr(), o=o.data_ptr(), stat=_ptr(stat),
                    stat_kind=_ptr(stat_kind), sink=_ptr(sink), q_gain=_ptr(q_gain), k_gain=_ptr(k_gain),
                    cos=_ptr(cos), sin=_ptr(sin), eps=float(eps), B=B, H=H, Tq=T, Tk=Tk, D=D, n=int(n),
@@ -479,8 +528,7 @@ def flash_attention_backward(q, k, v, o, d_o, stat, stat_kind, sink_logit=None, 
         d_o = torch.empty_strided(o.shape, o.stride(), dtype=o.dtype, device=o.device).copy_(d_o)
     sink = None
     if sink_logit is not None:
-        s = torch.as_tensor(sink_logit, dtype=torch.float32, device=q.device).reshape(-1)
-        sink = s.expand(H).contiguous() if s.numel() == 1 else s.contiguous()
+        sink = _sink_vector(sink_logit, H, q.device)
     dq, dk, dv = (torch.empty_strided(t.shape, t.stride(), dtype=t.dtype, device=t.device) for t in (q, k, v))
     dsink = torch.empty(H, dtype=torch.float32, device=q.device) if sink is not None else None
     if q.numel() == 0:
@@ -520,8 +568,7 @@ def decode_attention(q, k, v, sink_logit=None, *, n: int = 16, c: float = 8.0, o
     Tk = k.shape[2]
     sink = None
     if sink_logit is not None:
-        s = torch.as_tensor(sink_logit, dtype=torch.float32, device=q.device).reshape(-1)
-        sink = s.expand(H).contiguous() if s.numel() == 1 else s.contiguous()
+        sink = _sink_vector(sink_logit, H, q.device)
     q = q.contiguous()
     o = torch.empty((B, H, 1, D), dtype=q.dtype, device=q.device) if out is None else out
     a = L.DecodeArgs(q=q.data_ptr(), k=k.data_ptr(), v=v.data_ptr(), o=o.data_ptr(), sink=_ptr(sink),

@@ -153,24 +153,15 @@ class Prefill:
         B, T = tokens.shape
         d, H, D, f = cfg.d_model, cfg.n_heads, cfg.head_dim, cfg.d_ff
         x = ops.rms_norm(p["embed"][tokens].contiguous(), p["embed_gain"], cfg.eps).view(B * T, d)
-        attn_out = torch.empty((B, T, H, D), dtype=torch.bfloat16, device=self.device)
         if self.fused_proj:
             self.guard_words.zero_()
         if self.norm_in_weights:
-            # x stays the un-normalised residual stream; `ss` carries the row statistic of the next norm
-            ss = ops.row_sumsq(x)
-            for layer in range(cfg.n_layers):
-                qkv = ops.qkv_projection(x, p["w_qkv_t"][layer], H, T, self.cos_lp, self.sin_lp, p["q_gain"][layer],
-                                         p["k_gain"][layer], cfg.eps, cfg.attn_c, self.guard_words[layer],
-                                         row_ss=ss, guard_is_zero=True).view(B, T, 3, H, D)
-                q, k, v = (qkv[:, :, i].transpose(1, 2) for i in range(3))      # (B,H,T,D) views
-                ops.flash_attention(q, k, v, p["sink"][layer], kind="asinh", n=cfg.attn_n, c=cfg.attn_c, block=T,
-                                    range_guard=True, impl=self.impl, guard_words=self.guard_words[layer],
-                                    out=attn_out.transpose(1, 2))
-                x, ss = ops.resid_projection(attn_out.view(B * T, d), p["w_o_t"][layer], x, out=x)
-                ff = ops.glu_projection(x, p["w_gu_t"][layer], cfg.alu_beta, row_ss=ss, eps=cfg.eps)
-                x, ss = ops.resid_projection(ff, p["w_d_t"][layer], x, out=x)
-            return ops.rms_norm(x, p["final_gain"], cfg.eps).view(B, T, d)
+            # the norms as row scales inside the projections: five launches a block, all issued by one native call
+            return ops.prefill_blocks(x, p["w_qkv_t"], p["w_o_t"], p["w_gu_t"], p["w_d_t"], p["q_gain"], p["k_gain"],
+                                      p["sink"], p["final_gain"], self.cos_lp, self.sin_lp, self.guard_words, batch=B,
+                                      n_heads=H, eps=cfg.eps, alu_beta=cfg.alu_beta, attn_n=cfg.attn_n, attn_c=cfg.attn_c,
+                                      impl=self.impl).view(B, T, d)
+        attn_out = torch.empty((B, T, H, D), dtype=torch.bfloat16, device=self.device)
         for layer in range(cfg.n_layers):
             h = ops.rms_norm(x, p["ln1"][layer], cfg.eps)
             if self.fused_proj:

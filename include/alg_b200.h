@@ -453,6 +453,38 @@ ALG_API int alg_resid_proj_fwd(const alg_resid_proj_args* args, void* stream);
  * projection of a model (its input comes from the embedding's norm, not from a residual GEMM). */
 ALG_API int alg_row_sumsq(const void* x, int64_t rows, int d, int64_t ld_x, float* ss_out, void* stream);
 
+/* All blocks of a prefill and the final norm (src/algebraic/model.py:162-208) in one call: per block
+ * alg_qkv_proj_fwd, alg_attn_fwd (guarded, with the projection's maxima), alg_resid_proj_fwd, alg_glu_proj_fwd,
+ * alg_resid_proj_fwd, the norms as row scales; the same kernels with the same arguments as those calls made one by one.
+ * x: (B T, d) bf16 contiguous, the residual stream: the normalised embedding on entry, the last block's output on
+ * return.  out: (B T, d) bf16, normalised with final_gain.  Weights as their own entry points take them, stacked over
+ * L blocks and contiguous; the norms' gains are folded into w_qkv and w_gu.  guard: L records of 16 bytes, zeroed by
+ * the caller on this stream.  workspace: alg_prefill_blocks_workspace_bytes, 256-byte aligned. */
+typedef struct {
+  void* x;
+  void* out;
+  const void* w_qkv;       /* (L, 3 H D, d) */
+  const void* w_o;         /* (L, d, H D) */
+  const void* w_gu;        /* (L, 2 f, d), interleaved as for alg_glu_proj_fwd */
+  const void* w_d;         /* (L, d, f) */
+  const float* q_gain;     /* (L, D) or NULL */
+  const float* k_gain;     /* (L, D) or NULL */
+  const float* sink;       /* (L, H) or NULL */
+  const float* final_gain; /* (d) or NULL */
+  const void* cos;         /* (>= T, D / 2) bf16 */
+  const void* sin;
+  void* guard;
+  int L, B, T, H, D, d, f;
+  int attn_n;
+  float attn_c, eps, alu_beta;
+  int impl;
+  void* workspace;
+  size_t workspace_bytes;
+  int* status;             /* device int, may be NULL */
+} alg_prefill_blocks_args;
+ALG_API size_t alg_prefill_blocks_workspace_bytes(const alg_prefill_blocks_args* args);
+ALG_API int alg_prefill_blocks(const alg_prefill_blocks_args* args, void* stream);
+
 /* Backward of the Alg-CE head, first half: the logit gradient.  Replaces fused_head._bwd_kernel
  * (src/algebraic/kernels/fused_head.py:120-156), which also writes dz in bf16 and leaves
  * dh = dz . E and dE = dz^T . h to library matmuls (fused_head.py:194-216).
