@@ -408,9 +408,11 @@ struct Item {
 // KS = false is the kernel for lists without parts (every problem large enough to fill the GPU): the part
 // arithmetic and the partial epilogue are compiled out, which the head_dim-64 kernel with its 96 registers
 // per thread notices (5 % at the 125M layer shape).
-template <bool KS>
+// ONE: items of one query tile (see single_tiles below).
+template <bool KS, bool ONE>
 __device__ __forceinline__ bool item_at(const AttnParams& p, const ItemLists& lists, int k, Item& it) {
-  const int units = p.B * p.H, nblk = (p.Tq + 2 * BQ - 1) / (2 * BQ), G = int(gridDim.x);
+  constexpr int rows = ONE ? BQ : 2 * BQ;        // of an item
+  const int units = p.B * p.H, nblk = (p.Tq + rows - 1) / rows, G = int(gridDim.x);
   int idx, part = 0, parts = 1;
   it.slot = 0;
   if (lists.listed) {
@@ -426,6 +428,12 @@ __device__ __forceinline__ bool item_at(const AttnParams& p, const ItemLists& li
   }
   const int blk = nblk - 1 - idx / units, bh = idx % units;
   it.b = bh / p.H; it.h = bh % p.H;
+  if (ONE) {                                     // the item's one tile is query tile 1; query tile 0 has no part in the launch
+    it.row0 = (blk - 1) * BQ;
+    it.k0 = 0; it.n1 = blk + 1; it.n0 = 0;
+    it.diag = it.first = true; it.partial = false;
+    return true;
+  }
   it.row0 = blk * 2 * BQ;
   const int steps = 2 * blk + 2;                 // key tiles needed by query tile 1 (tile 0: one fewer)
   it.k0 = steps * part / parts;
@@ -538,13 +546,14 @@ struct ScaleSplit {
 // 128 columns, the first 64 the bf16 rounding of the fp32 values (hi) and the other 64 what it left
 // over (lo); every product is issued as hi.hi + hi.lo + lo.hi into the same accumulator, for the
 // scores and - with the weights split the same way - for the output, which is written as fp32.
-template <int D, int LOG2N, int SPLIT, bool SHIFT, bool F32 = false, bool KS = false>
+template <int D, int LOG2N, int SPLIT, bool SHIFT, bool F32 = false, bool KS = false, bool ONE = false>
 __global__ void __launch_bounds__(nthreads<SPLIT>(), 1)
 attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ AttnParams p, const ScaleSplit sc,
                const __grid_constant__ ItemLists lists) {
   using C = Cfg<D>;
   static_assert(!F32 || (D == 128 && SPLIT == 1 && !SHIFT), "the fp32 mode: hi|lo tiles of head_dim 64, unshifted form");
+  static_assert(!ONE || (!SHIFT && !F32 && !KS), "items of one query tile are whole items of the unshifted bf16 form");
   static_assert(!KS || (!SHIFT && !F32), "items are split along the keys in the unshifted bf16 form only");
   constexpr int DV = F32 ? 64 : D;                  // output columns
   // head_dim 64, unshifted, split weight groups: P_w has tensor-memory columns of its own and S_w is re-issued
@@ -606,7 +615,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       tma_prefetch_desc(&tm_q); tma_prefetch_desc(&tm_k); tma_prefetch_desc(&tm_v);
       bool ok = true;
       RingCursor<C::NKV> cur;                       // runs on over all items
-      for (int k = 0; ok && item_at<KS>(p, lists, k, it); ++k) {
+      for (int k = 0; ok && item_at<KS, ONE>(p, lists, k, it); ++k) {
         auto load_kv = [&](int idx) {               // K_0, V_0, K_1, V_1, ... of this item
           const int buf = cur.slot;
           if (!bw.wait(&ctl->kv_empty[buf], cur.phase ^ 1u)) return false;
@@ -619,6 +628,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           return true;
         };
         auto load_q = [&](int w) {                  // after the previous item's last S_w has read the tile
+          if (ONE && w == 0) return true;
           if (k > 0 && !bw.wait(&ctl->q_free[w], (k - 1) & 1u)) return false;
           mbar_arrive_expect_tx(&ctl->q_full[w], C::TILE_BYTES);
           for (int pn = 0; pn < C::PANELS; ++pn)
@@ -716,11 +726,11 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     const long long t_begin = clock64();
 #endif
     bool ok = true;
-    for (int k = 0; ok && item_at<KS>(p, lists, k, it); ++k) {
+    for (int k = 0; ok && item_at<KS, ONE>(p, lists, k, it); ++k) {
       const int n0 = it.n0, n1 = it.n1;
-      if (!wait_all(&ctl->q_ready[0], k & 1u) || !kv_wait(cur)) { ok = false; break; }
+      if ((!ONE && !wait_all(&ctl->q_ready[0], k & 1u)) || !kv_wait(cur)) { ok = false; break; }
       tc_fence_after();
-      if (elect_one()) { issue_s(0, cur.slot); umma_commit(&ctl->s_full[0]); }
+      if (!ONE && elect_one()) { issue_s(0, cur.slot); umma_commit(&ctl->s_full[0]); }
       __syncwarp();
       if (!wait_all(&ctl->q_ready[1], k & 1u)) { ok = false; break; }
       tc_fence_after();
@@ -810,8 +820,8 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     // and release the tile to the MMA warp.
     const __nv_bfloat162 f2 = __float2bfloat162_rn(sc.pow2);
     bool ok = true;
-    for (int k = 0; ok && item_at<KS>(p, lists, k, it); ++k) {
-      for (int w = 0; w < 2 && ok; ++w) {
+    for (int k = 0; ok && item_at<KS, ONE>(p, lists, k, it); ++k) {
+      for (int w = ONE ? 1 : 0; w < 2 && ok; ++w) {
         if (!bw.wait(&ctl->q_full[w], k & 1u)) { ok = false; break; }
         if (sc.pow2 != 1.0f) {
           uint4* tile = reinterpret_cast<uint4*>(smem + C::Q_OFF + w * C::TILE_BYTES);
@@ -844,7 +854,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     const int r = quarter * 32 + lane;              // row inside the query tile
     const uint32_t lane_sel = uint32_t(quarter * 32) << 16;
     const uint32_t s_taddr = tmem_base + lane_sel + C::S_COL + w * 128;
-    bool ok = true;
+    bool ok = !(ONE && w == 0);
     int tiles_before = 0;                           // score tiles of this group in earlier items
     // One thread per group passes on what the arrival of scores implies.  The tensor pipe runs the
     // MMA thread's instructions in order, so "S_w(j) is there" means every product issued before it
@@ -860,7 +870,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
 #ifdef ALG_ATTN_TIMING
     const long long t_begin = clock64();
 #endif
-    for (int k = 0; ok && item_at<KS>(p, lists, k, it); ++k) {
+    for (int k = 0; ok && item_at<KS, ONE>(p, lists, k, it); ++k) {
       const int nk = (w == 0) ? it.n0 : it.n1;
       const int last_masked = (!KS || it.diag) ? nk - 1 : -1; // the tile that holds this query tile's diagonal (last part of an item only)
       float l = 0.f;                                // the sink's weight, fetched while the first scores are computed
@@ -964,7 +974,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         }
       }
       tc_fence_after();
-      item_at<KS>(p, lists, k, it);                            // recomputed: nothing of it stays live over the tile loop
+      item_at<KS, ONE>(p, lists, k, it);                            // recomputed: nothing of it stays live over the tile loop
       l += part;                                    // shifted form: the last tile's sums (already at the final maximum)
       const float inv = 1.0f / l;
       const int row = it.row0 + w * BQ + r;
@@ -1056,12 +1066,12 @@ constexpr int MIN_PART_TILES = 32, MAX_SPLIT_ENTRIES = 512;
 struct DealEntry { int cost; uint16_t code; };
 
 // the entries for parts of about `target` tiles (0: whole items); returns their number, or -1 if they do not fit
-int deal_entries(DealEntry* entry, int units, int nblk, int target, int* parts_total) {
+int deal_entries(DealEntry* entry, int units, int nblk, bool single, int target, int* parts_total) {
   const int items = units * nblk;
   int entries = 0;
   *parts_total = 0;
   for (int i = 0; i < items; ++i) {
-    const int blk = nblk - 1 - i / units, cost = 4 * blk + 3, steps = 2 * blk + 2;
+    const int blk = nblk - 1 - i / units, cost = single ? blk + 1 : 4 * blk + 3, steps = 2 * blk + 2;
     int parts = 1;
     if (target > 0 && cost > target) {
       parts = (cost + target - 1) / target;
@@ -1071,7 +1081,7 @@ int deal_entries(DealEntry* entry, int units, int nblk, int target, int* parts_t
     if (entries + parts > (target > 0 ? MAX_SPLIT_ENTRIES : MAX_LISTED)) return -1;
     for (int pt = 0; pt < parts; ++pt) {
       const int k0 = steps * pt / parts, k1 = steps * (pt + 1) / parts;
-      entry[entries].cost = 2 * (k1 - k0) - (pt == parts - 1 ? 1 : 0);
+      entry[entries].cost = parts == 1 ? cost : 2 * (k1 - k0) - (pt == parts - 1 ? 1 : 0);
       entry[entries].code = uint16_t(i | (pt << 10) | ((parts - 1) << 13));
       ++entries;
     }
@@ -1099,7 +1109,7 @@ int deal_greedy(const DealEntry* entry, int entries, int grid, uint16_t* owner, 
   return worst;
 }
 
-int deal_items(ItemLists* out, int units, int nblk, int grid, bool split) {
+int deal_items(ItemLists* out, int units, int nblk, int grid, bool split, bool single) {
   const int items = units * nblk;
   out->listed = 0;
   if (items > MAX_LISTED || grid > MAX_LIST_CTAS) return 0;
@@ -1111,16 +1121,16 @@ int deal_items(ItemLists* out, int units, int nblk, int grid, bool split) {
   const int share = int((total + grid - 1) / grid), heaviest = 4 * (nblk - 1) + 3;
   int best_target = 0, parts_total = 0;
   if (split && 2 * heaviest > 3 * share) {
-    int entries = deal_entries(entry, units, nblk, 0, &parts_total);
+    int entries = deal_entries(entry, units, nblk, single, 0, &parts_total);
     int best_score = deal_greedy(entry, entries, grid, owner, count);
     for (int target = MIN_PART_TILES; target < heaviest; target += (target < 64 ? 8 : (target < 128 ? 16 : 64))) {
-      entries = deal_entries(entry, units, nblk, target, &parts_total);
+      entries = deal_entries(entry, units, nblk, single, target, &parts_total);
       if (entries < 0 || parts_total == 0) continue;
       const int score = deal_greedy(entry, entries, grid, owner, count) + parts_total / 10 + 6;
       if (score < best_score) { best_score = score; best_target = target; }
     }
   }
-  const int entries = deal_entries(entry, units, nblk, best_target, &parts_total);
+  const int entries = deal_entries(entry, units, nblk, single, best_target, &parts_total);
   deal_greedy(entry, entries, grid, owner, count);
   out->start[0] = 0;
   for (int c = 0; c < grid; ++c) out->start[c + 1] = uint16_t(out->start[c] + count[c]);
@@ -1131,20 +1141,21 @@ int deal_items(ItemLists* out, int units, int nblk, int grid, bool split) {
   return parts_total;
 }
 
-// The deal depends on four integers only: keep the last few (a launch path must stay cheap, and a call asks
+// The deal depends on five integers only: keep the last few (a launch path must stay cheap, and a call asks
 // twice - once for the workspace size, with splitting, once at the launch, with or without).
-struct Dealt { int units, nblk, grid, split, parts; ItemLists lists; };
-const Dealt& dealt_for(int units, int nblk, int grid, bool split) {
+struct Dealt { int units, nblk, grid, split, single, parts; ItemLists lists; };
+const Dealt& dealt_for(int units, int nblk, int grid, bool split, bool single) {
   constexpr int KEPT = 16;
   static thread_local Dealt kept[KEPT];
   static thread_local int used = 0, next = 0;
   for (int i = 0; i < used; ++i)
-    if (kept[i].units == units && kept[i].nblk == nblk && kept[i].grid == grid && kept[i].split == int(split)) return kept[i];
+    if (kept[i].units == units && kept[i].nblk == nblk && kept[i].grid == grid && kept[i].split == int(split) &&
+        kept[i].single == int(single)) return kept[i];
   Dealt& d = kept[next];
   next = (next + 1) % KEPT;
   if (used < KEPT) ++used;
-  d.units = units; d.nblk = nblk; d.grid = grid; d.split = int(split);
-  d.parts = deal_items(&d.lists, units, nblk, grid, split);
+  d.units = units; d.nblk = nblk; d.grid = grid; d.split = int(split); d.single = int(single);
+  d.parts = deal_items(&d.lists, units, nblk, grid, split, single);
   return d;
 }
 
@@ -1222,18 +1233,33 @@ int make_qkv_map(CUtensorMap* tm, const void* base, const Strides3& s, int B, in
   return make_tmap_bf16(tm, base, 4, dims, strides, box, true);
 }
 
-template <int D, int LOG2N, int SPLIT, bool SHIFT, bool F32, bool KS>
+template <int D, int LOG2N, int SPLIT, bool SHIFT, bool F32, bool KS, bool ONE>
 int launch_kernel(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const AttnParams& p, const ScaleSplit& sc,
                   const ItemLists& lists, int grid, cudaStream_t stream) {
-  auto kern = attn_tc_kernel<D, LOG2N, SPLIT, SHIFT, F32, KS>;
+  auto kern = attn_tc_kernel<D, LOG2N, SPLIT, SHIFT, F32, KS, ONE>;
   static PerDeviceOnce configured;
   if (int rc = configured.run([&] { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_bytes<D>())); })) return rc;
   ALG_CUDA_TRY(launch_dependent(kern, dim3(grid), dim3(nthreads<SPLIT>()), smem_bytes<D>(), stream, tq, tk, tv, p, sc, lists));
   return ALG_OK;
 }
 
+// Items of one query tile or of two.  Two tiles share their K and V tiles and keep the pipes busier, but a step of
+// both takes longer than a step of one: where the longest item sets the time, one tile ends sooner.  The estimate is
+// the longest CTA's steps (the longest item, or an even share and one for the uneven deal) times the time of a step, one
+// tile's being 0.75 to 0.9 of two tiles'.  Measured, two -> one: (1,12,613,64) 14.8 -> 10.9 us, (1,12,2048,64) 31.9 -> 24.6,
+// (1,16,613,128) 17.5 -> 14.3, (1,16,2048,128) 35.9 -> 33.3; (2,12,2048,64) 32.0 -> 38.2, (16,12,1024,64) 61 -> 84.
+template <int D>
+bool single_tiles(int units, int T, int grid) {
+  const int64_t nq = (T + BQ - 1) / BQ, nblk = (nq + 1) / 2;
+  if (units * nq > MAX_LISTED) return false;
+  const int64_t one = std::max(nq, (units * nq * (nq + 1) / 2 + grid - 1) / grid + 1);
+  const int64_t two = std::max(2 * nblk, (units * nblk * (nblk + 1) + grid - 1) / grid);
+  return one * (D == 64 ? 90 : 95) < two * 100;
+}
+
 template <int D, int LOG2N, int SPLIT, bool SHIFT, bool F32 = false>
-int launch_dns(const AttnParams& p, cudaStream_t stream) {
+int launch_dns(const AttnParams& params, cudaStream_t stream) {
+  AttnParams p = params;
   CUtensorMap tq, tk, tv;
   if (int rc = make_qkv_map(&tq, p.q, p.qs, p.B, p.H, p.Tq, D)) return rc;
   if (int rc = make_qkv_map(&tk, p.k, p.ks, p.B, p.H, p.Tk, D)) return rc;
@@ -1254,13 +1280,21 @@ int launch_dns(const AttnParams& p, cudaStream_t stream) {
   // short problems: long items are cut along the keys when the caller's workspace has room for the parts' slots
   static const bool never_split = getenv("ALG_ATTN_NO_KEY_SPLIT") != nullptr;      // measurement aid
   const bool may_split = !SHIFT && !F32 && p.split_ws != nullptr && !never_split;
-  const Dealt* dealt = &dealt_for(units, nblk, grid, may_split);
-  if (dealt->parts > 0 && int(dealt->lists.start[grid]) > p.split_slots) dealt = &dealt_for(units, nblk, grid, false);
+  const Dealt* dealt = &dealt_for(units, nblk, grid, may_split, false);
+  if (dealt->parts > 0 && int(dealt->lists.start[grid]) > p.split_slots) dealt = &dealt_for(units, nblk, grid, false, false);
+  const bool single = !SHIFT && !F32 && dealt->parts == 0 && single_tiles<D>(units, p.Tq, grid);
+  const int tiles = (p.Tq + BQ - 1) / BQ;
+  if (single) dealt = &dealt_for(units, tiles, grid, false, true);
+  const ItemLists& lists = dealt->lists;
+  int rc;
   if constexpr (!SHIFT && !F32) {
-    if (dealt->parts > 0) {
-      if (int rc = launch_kernel<D, LOG2N, SPLIT, SHIFT, F32, true>(tq, tk, tv, p, sc, dealt->lists, grid, stream)) return rc;
-    } else if (int rc = launch_kernel<D, LOG2N, SPLIT, SHIFT, F32, false>(tq, tk, tv, p, sc, dealt->lists, grid, stream)) return rc;
-  } else if (int rc = launch_kernel<D, LOG2N, SPLIT, SHIFT, F32, false>(tq, tk, tv, p, sc, dealt->lists, grid, stream)) return rc;
+    if (dealt->parts > 0) rc = launch_kernel<D, LOG2N, SPLIT, SHIFT, F32, true, false>(tq, tk, tv, p, sc, lists, grid, stream);
+    else if (single) rc = launch_kernel<D, LOG2N, SPLIT, SHIFT, F32, false, true>(tq, tk, tv, p, sc, lists, grid, stream);
+    else rc = launch_kernel<D, LOG2N, SPLIT, SHIFT, F32, false, false>(tq, tk, tv, p, sc, lists, grid, stream);
+  } else {
+    rc = launch_kernel<D, LOG2N, SPLIT, SHIFT, F32, false, false>(tq, tk, tv, p, sc, lists, grid, stream);
+  }
+  if (rc) return rc;
   if (dealt->parts > 0) {
     const int entries = int(dealt->lists.start[grid]);
     ALG_CUDA_TRY(launch_dependent(attn_split_combine_kernel<D>, dim3(entries, 8), dim3(256), 0, stream, dealt->lists, p, entries, sc.inv_mn));
@@ -1383,7 +1417,7 @@ int attn_tcgen05_grid(const AttnParams& p) {
 size_t attn_tcgen05_split_bytes(const AttnParams& p) {
   if (p.D != 64 && p.D != 128) return 0;
   const int units = p.B * p.H, nblk = (p.Tq + 2 * BQ - 1) / (2 * BQ), grid = attn_tcgen05_grid(p);
-  const Dealt& d = dealt_for(units, nblk, grid, true);
+  const Dealt& d = dealt_for(units, nblk, grid, true, false);
   return d.parts > 0 ? size_t(d.lists.start[grid]) * 2 * BQ * (p.D + 4) * sizeof(float) : 0;
 }
 
