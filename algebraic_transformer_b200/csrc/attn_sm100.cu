@@ -576,6 +576,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   // each form runs only when it is the one called for: under a guard the unshifted kernel leaves when the
   // guard failed and the shifted kernel leaves when it held
   if ((ctl->shift_mode != 0) != SHIFT) return;
+  if (p.announce) griddep_launch();
 
   if (threadIdx.x == 0) {
     for (int w = 0; w < 2; ++w) { mbar_init(&ctl->q_full[w], 1); mbar_init(&ctl->q_ready[w], 1); mbar_init(&ctl->q_free[w], 1); }
@@ -1285,6 +1286,7 @@ int launch_dns(const AttnParams& params, cudaStream_t stream) {
   const bool single = !SHIFT && !F32 && dealt->parts == 0 && single_tiles<D>(units, p.Tq, grid);
   const int tiles = (p.Tq + BQ - 1) / BQ;
   if (single) dealt = &dealt_for(units, tiles, grid, false, true);
+  p.announce = units * (single ? tiles : nblk) * 2 <= grid;
   const ItemLists& lists = dealt->lists;
   int rc;
   if constexpr (!SHIFT && !F32) {

@@ -153,10 +153,14 @@ __device__ __forceinline__ bool guard_in_range(const GuardWords* g, float bound_
 // after that whole kernel has drained; griddep_wait() in it returns once that kernel has finished
 // and its writes are visible (a no-op in a kernel launched the plain way).  So a kernel's set-up
 // (barriers, tensor memory, descriptor prefetch) and its launch latency overlap the tail of the one
-// before.  The earlier kernels do not announce themselves early (griddepcontrol.launch_dependents):
+// before.  Kernels of more than one round do not announce themselves early (griddepcontrol.launch_dependents):
 // measured on the prefill step, CTAs that sit waiting beside a running kernel cost a long step 1-2 %,
 // while leaving it to each CTA's exit keeps the whole gain of the short steps (3 % at 2048 tokens).
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Lets the next dependent kernel's CTAs move onto SMs this grid leaves free, once every CTA has said so (or left).  Called
+// after griddep_wait(): what the kernels before this one wrote is then complete when the next one's set-up starts.
+__device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // Launch `kern` so that it may start before the kernel ahead of it in `stream` has finished
 // (programmatic dependent launch); the kernel itself calls griddep_wait() before it touches

@@ -64,6 +64,7 @@ int launch_scale_bf16(const void* src, const float* scale, void* dst, int dst_dt
 
 // ---- attention ----------------------------------------------------------------------
 struct AttnParams {
+  int announce;            // tcgen05 kernel: items leave SMs free, let the next kernel's CTAs in early
   const void* q;
   const void* k;
   const void* v;
@@ -165,6 +166,7 @@ int launch_attn_bwd_tcgen05(const AttnBwdParams& p, cudaStream_t stream);
 
 // ---- proj_sm100.cu: projection GEMMs with fused epilogues -------------------------------
 struct ProjParams {
+  int announce;            // every tile has a CTA of its own: let the next kernel's CTAs in beside this one's
   int M, K, N;             // activations (M, K), weights (N, K), both K-major bf16
   int64_t ld_x;
   __nv_bfloat16* out;

@@ -43,7 +43,7 @@ namespace {
 using namespace sm100;
 
 constexpr int BM = 128, BK = 64, UMMA_K = 16;   // BM: accumulator rows of one CTA
-constexpr int BN_MAX = 256;                      // accumulator tile width: 256, or 128 for the residual GEMM on few rows
+constexpr int BN_MAX = 256;                      // accumulator tile width: 256, or 128 where that fills the chip better
 constexpr int A_BYTES = BM * BK * 2;
 constexpr int NTHREADS = 320, EPI_WARPS = 8;
 constexpr uint32_t TMEM_COLS = 512;
@@ -362,24 +362,25 @@ __device__ __forceinline__ void glu16(const uint32_t* gu, float beta, float tau_
   }
 }
 
-// 64 output features of one row: gate columns from t_gate, up columns from t_up
+// NF (64 or 32) output features of one row: gate columns from t_gate, up columns from t_up
+template <int NF>
 __device__ __forceinline__ void glu_cols(const ProjParams& p, uint32_t t_gate, uint32_t t_up, const WarpOut& wo, int lane,
                                          int col, float tau_row) {
-  uint32_t a[32], b[32], o[32];
+  uint32_t a[32], b[32], o[32] = {};
   tmem_ld_32x16(t_gate, a);
   tmem_ld_32x16(t_up, a + 16);
 #pragma unroll
-  for (int c = 0; c < 4; ++c) {
+  for (int c = 0; c < NF / 16; ++c) {
     uint32_t* cur = (c & 1) ? b : a;
     uint32_t* nxt = (c & 1) ? a : b;
     tmem_ld_wait_for(cur);
-    if (c + 1 < 4) {
+    if (c + 1 < NF / 16) {
       tmem_ld_32x16(t_gate + (c + 1) * 16, nxt);
       tmem_ld_32x16(t_up + (c + 1) * 16, nxt + 16);
     }
     glu16(cur, p.beta, tau_row, o + 8 * c);
   }
-  store_rows64(wo, lane, o, col);
+  store_rows64(wo, lane, o, col, NF);
 }
 
 template <int EPI, int D, int BN, int CG>
@@ -422,6 +423,7 @@ proj_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
   // Launched as a programmatic dependent: everything above overlapped the tail of the kernel ahead in the
   // stream; from here on its results are complete.
   griddep_wait();
+  if (p.announce) griddep_launch();
   const uint32_t tmem_base = ctl->tmem_base;
   const BoundedWait bw{&ctl->abort_flag, 1000000000ull};
   const int tiles_n = (p.N + BN - 1) / BN;
@@ -445,7 +447,13 @@ proj_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
             tma_load_2d_pair(dst + A_BYTES, &tm_w, bar, kb * BK, col);
           } else {
             tma_load_2d(dst, &tm_x, &ctl->full[stage], kb * BK, row);
-            tma_load_2d(dst + A_BYTES, &tm_w, &ctl->full[stage], kb * BK, col);
+            if (EPI == EPI_GLU && BN == 128) {           // 64 gate rows and the matching 64 up rows of a 128 + 128 block
+              const int gate = u % tiles_n / 2 * 256 + u % tiles_n % 2 * 64;
+              tma_load_2d(dst + A_BYTES, &tm_w, &ctl->full[stage], kb * BK, gate);
+              tma_load_2d(dst + A_BYTES + 64 * BK * 2, &tm_w, &ctl->full[stage], kb * BK, gate + 128);
+            } else {
+              tma_load_2d(dst + A_BYTES, &tm_w, &ctl->full[stage], kb * BK, col);
+            }
           }
           if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
@@ -501,7 +509,7 @@ proj_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
       constexpr int TQ = (EPI == EPI_QKV) ? D / 4 : 1;
       uint32_t tc[TQ], ts[TQ];
       const int hd = p.H * D;
-      if (EPI == EPI_QKV && (n * BN + half * 128) / hd < 2) {   // kinds only grow along a tile: q/k present
+      if (EPI == EPI_QKV && (n * BN + half * (BN / 2)) / hd < 2) {   // kinds only grow along a tile: q/k present
         const int t = live ? row % p.T : 0;
         const uint4* ct = reinterpret_cast<const uint4*>(p.cos + int64_t(t) * (D / 2));
         const uint4* st = reinterpret_cast<const uint4*>(p.sin + int64_t(t) * (D / 2));
@@ -526,8 +534,8 @@ proj_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
       const WarpOut wo{stage, p.out + int64_t(wrow) * p.ld_out, p.ld_out, wrows};
       if (EPI == EPI_QKV) {
 #pragma unroll 1
-        for (int hh = 0; hh < 128 / D; ++hh) {
-          const int lcol = half * 128 + hh * D;          // column inside the tile
+        for (int hh = 0; hh < BN / 2 / D; ++hh) {
+          const int lcol = half * (BN / 2) + hh * D;     // column inside the tile
           const int gcol = n * BN + lcol;                // output feature
           if (gcol >= p.N) break;
           qkv_head<D>(p, s_gain, tbuf + lcol, gcol / hd, tc, ts, wo, lane, gcol, live, tau_row, best_q, best_k, best_v);
@@ -557,9 +565,9 @@ proj_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
         }
         if (p.ss_out != nullptr && live) p.ss_out[int64_t(n * 2 + half) * p.M + row] = ss;
       } else {
-        const int fcol = n * 128 + half * 64;            // output feature of this thread's first column
+        const int fcol = n * (BN / 2) + half * (BN / 4); // output feature of this thread's first column
         if (fcol < p.f)
-          glu_cols(p, tbuf + half * 64, tbuf + 128 + half * 64, wo, lane, fcol, tau_row);
+          glu_cols<BN / 4>(p, tbuf + half * (BN / 4), tbuf + BN / 2 + half * (BN / 4), wo, lane, fcol, tau_row);
       }
       tc_fence_before();
       __syncwarp();
@@ -609,23 +617,168 @@ int launch_variant(const CUtensorMap& tm_x, const CUtensorMap& tm_w, const ProjP
   return ALG_OK;
 }
 
-template <int CG>
-int launch_cg(const CUtensorMap& tm_x, const CUtensorMap& tm_w, const ProjParams& p, int epi, int bn, int grid, cudaStream_t stream) {
-  if (epi == EPI_RESID) {
-    if constexpr (CG == 1) {
-      if (bn == 128) return launch_variant<EPI_RESID, 64, 128, 1>(tm_x, tm_w, p, grid, stream);
-    }
-    return launch_variant<EPI_RESID, 64, 256, CG>(tm_x, tm_w, p, grid, stream);
+template <int BN, int CG>
+int launch_tile(const CUtensorMap& tm_x, const CUtensorMap& tm_w, const ProjParams& p, int epi, int grid, cudaStream_t stream) {
+  if (epi == EPI_RESID) return launch_variant<EPI_RESID, 64, BN, CG>(tm_x, tm_w, p, grid, stream);
+  if (epi == EPI_GLU) return launch_variant<EPI_GLU, 64, BN, CG>(tm_x, tm_w, p, grid, stream);
+  if (epi == EPI_QKV && p.D == 64) return launch_variant<EPI_QKV, 64, BN, CG>(tm_x, tm_w, p, grid, stream);
+  if constexpr (BN == 256) {
+    if (epi == EPI_DZ) return launch_variant<EPI_DZ, 64, BN, CG>(tm_x, tm_w, p, grid, stream);
+    return launch_variant<EPI_QKV, 128, BN, CG>(tm_x, tm_w, p, grid, stream);
   }
-  if (epi == EPI_GLU) return launch_variant<EPI_GLU, 64, 256, CG>(tm_x, tm_w, p, grid, stream);
-  if (epi == EPI_DZ) return launch_variant<EPI_DZ, 64, 256, CG>(tm_x, tm_w, p, grid, stream);
-  return p.D == 64 ? launch_variant<EPI_QKV, 64, 256, CG>(tm_x, tm_w, p, grid, stream)
-                   : launch_variant<EPI_QKV, 128, 256, CG>(tm_x, tm_w, p, grid, stream);
+  set_error("internal: no narrow tile for this projection");
+  return ALG_ERR_UNSUPPORTED;
+}
+
+// ---- residual GEMM on few rows: the tile's K cut over a cluster ---------------------------------
+// A 613 x 768 output is 30 tiles of 128 x 128, so most SMs idle while 30 of them walk the whole of K (32 ring
+// steps for the 125M model's down-projection).  Here S CTAs of a cluster each take a 1 / S of K, leave
+// their fp32 partial tile in their own shared memory, and each adds up 128 / S rows over the cluster through
+// distributed shared memory, in rank order (repeatable), then applies the residual epilogue with a warp
+// per row: whole lines, no staging.  One tile per cluster, not persistent.
+template <int S>
+__global__ void __launch_bounds__(NTHREADS, 1)
+resid_split_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w, const ProjParams p) {
+  constexpr int BN = 128, STAGES = 6, STAGE_BYTES = A_BYTES + BN * BK * 2, ROWS = BM / S, RPW = ROWS / EPI_WARPS;
+  static_assert(STAGES * STAGE_BYTES == RING_BYTES && BM * BN * 4 <= RING_BYTES, "the ring, and the partial tile in its place");
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  Control* ctl = reinterpret_cast<Control*>(smem + RING_BYTES);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = int(cluster_rank()), tile = blockIdx.x / S;
+  const int tiles_n = (p.N + BN - 1) / BN, m = tile / tiles_n, n = tile % tiles_n;
+  const int kblocks = p.K / BK, kb0 = kblocks * rank / S, nkb = kblocks * (rank + 1) / S - kb0;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) { mbar_init(&ctl->full[s], 1); mbar_init(&ctl->empty[s], 1); }
+    mbar_init(&ctl->tfull[0], 1);
+    ctl->abort_flag = 0;
+    fence_barrier_init();
+    tma_prefetch_desc(&tm_x);
+    tma_prefetch_desc(&tm_w);
+  }
+  if (warp == 1) {
+    tmem_alloc(&ctl->tmem_base, BN);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  griddep_wait();
+  if (p.announce) griddep_launch();
+  const uint32_t tmem_base = ctl->tmem_base;
+  const BoundedWait bw{&ctl->abort_flag, 1000000000ull};
+  // this thread's share of the epilogue: RPW rows, four columns of each
+  const int col = n * BN + lane * 4, lrow0 = rank * ROWS + (warp - 2) * RPW;
+  uint2 res[RPW];
+
+  if (warp == 0) {
+    if (lane == 0) {
+      for (int i = 0; i < nkb; ++i) {
+        const int stage = i % STAGES;
+        if (!bw.wait(&ctl->empty[stage], ((i / STAGES) & 1) ^ 1)) break;
+        unsigned char* dst = smem + size_t(stage) * STAGE_BYTES;
+        mbar_arrive_expect_tx(&ctl->full[stage], STAGE_BYTES);
+        tma_load_2d(dst, &tm_x, &ctl->full[stage], (kb0 + i) * BK, m * BM);
+        tma_load_2d(dst + A_BYTES, &tm_w, &ctl->full[stage], (kb0 + i) * BK, n * BN);
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    constexpr uint32_t IDESC = make_idesc_bf16(BM, BN, 0, 0);
+    const uint32_t a_lo0 = sw128_desc_lo(smem_u32(smem), 16), b_lo0 = sw128_desc_lo(smem_u32(smem) + A_BYTES, 16);
+    for (int i = 0; i < nkb; ++i) {
+      const int stage = i % STAGES;
+      if (__all_sync(0xffffffffu, bw.wait(&ctl->full[stage], (i / STAGES) & 1)) == 0) break;
+      tc_fence_after();
+      if (elect_one()) {
+        const uint32_t a_lo = a_lo0 + stage * (STAGE_BYTES >> 4), b_lo = b_lo0 + stage * (STAGE_BYTES >> 4);
+#pragma unroll
+        for (int k = 0; k < BK / UMMA_K; ++k)
+          umma_f16_ss_parts(tmem_base, a_lo + k * (UMMA_K * 2 >> 4), SW128_DESC_HI, b_lo + k * (UMMA_K * 2 >> 4), SW128_DESC_HI,
+                            IDESC, (i | k) != 0 ? 1u : 0u);
+        umma_commit(&ctl->empty[stage]);
+        if (i == nkb - 1) umma_commit(&ctl->tfull[0]);
+      }
+      __syncwarp();
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < RPW; ++i) {              // the residual, while the partial sums form
+      const int row = m * BM + lrow0 + i;
+      res[i] = make_uint2(0u, 0u);
+      if (row < p.M && col < p.N) res[i] = *reinterpret_cast<const uint2*>(p.resid + int64_t(row) * p.ld_resid + col);
+    }
+    // the partial tile -> shared memory, where the ring was (all loads and products are done once tfull is
+    // complete); 16-byte chunks XOR-swizzled by row within groups of eight
+    const bool done = bw.wait(&ctl->tfull[0], 0);
+    if (__all_sync(0xffffffffu, done)) {
+      tc_fence_after();
+      const int quarter = warp & 3, half = (warp - 2) >> 2, row = quarter * 32 + lane;
+      float4* dst = reinterpret_cast<float4*>(smem + row * BN * 4);
+      uint32_t r[2][32];
+      tmem_ld_32x32(tmem_base + (uint32_t(quarter * 32) << 16) + half * 64, r[0]);
+      tmem_ld_32x32(tmem_base + (uint32_t(quarter * 32) << 16) + half * 64 + 32, r[1]);
+      tmem_ld_wait_for(r[0]);
+      tmem_ld_wait_for(r[1]);
+#pragma unroll
+      for (int c = 0; c < 16; ++c) {
+        const uint32_t* v = r[c >> 3] + (c & 7) * 4;
+        dst[(half * 16 + c) ^ (row & 7)] = make_float4(__uint_as_float(v[0]), __uint_as_float(v[1]), __uint_as_float(v[2]), __uint_as_float(v[3]));
+      }
+      tc_fence_before();
+    }
+    __syncwarp();
+  }
+  cluster_sync_all();                            // every partial tile is in place
+  if (warp >= 2) {
+#pragma unroll
+    for (int i = 0; i < RPW; ++i) {
+      const int lrow = lrow0 + i, row = m * BM + lrow;
+      const uint32_t at = smem_u32(smem) + lrow * BN * 4 + ((uint32_t(lane) ^ uint32_t(lrow & 7)) << 4);
+      float4 part[S];
+#pragma unroll
+      for (int s = 0; s < S; ++s) part[s] = ld_cluster_f4(at, s);
+      float4 v = part[0];
+#pragma unroll
+      for (int s = 1; s < S; ++s) { v.x += part[s].x; v.y += part[s].y; v.z += part[s].z; v.w += part[s].w; }
+      const uint32_t y0 = pack_bf16(pair_lo(res[i].x) + v.x, pair_hi(res[i].x) + v.y);
+      const uint32_t y1 = pack_bf16(pair_lo(res[i].y) + v.z, pair_hi(res[i].y) + v.w);
+      const bool live = row < p.M && col < p.N;
+      if (live) *reinterpret_cast<uint2*>(p.out + int64_t(row) * p.ld_out + col) = make_uint2(y0, y1);
+      float ss = live ? pair_lo(y0) * pair_lo(y0) + pair_hi(y0) * pair_hi(y0) + pair_lo(y1) * pair_lo(y1) + pair_hi(y1) * pair_hi(y1) : 0.f;
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);   // the 64 columns of one partial
+      if (p.ss_out != nullptr && row < p.M && (lane & 15) == 0) p.ss_out[int64_t(n * 2 + (lane >> 4)) * p.M + row] = ss;
+    }
+  }
+  __syncwarp();
+  cluster_sync_all();                            // the others may still be reading this CTA's tile
+  if (ctl->abort_flag != 0 && threadIdx.x == 0) {
+    if (p.status != nullptr) atomicExch(p.status, ALG_DEV_TIMEOUT);
+    const uint64_t t0 = global_timer_ns();       // let issued loads land before shared memory is released
+    while (global_timer_ns() - t0 < 200000ull) { }
+  }
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, BN);
+  }
+}
+
+template <int S>
+int launch_split(const CUtensorMap& tm_x, const CUtensorMap& tm_w, const ProjParams& p, int tiles, cudaStream_t stream) {
+  auto kern = resid_split_kernel<S>;
+  static PerDeviceOnce configured;
+  if (int rc = configured.run([&] { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(SMEM_BYTES)); })) return rc;
+  ALG_CUDA_TRY(launch_dependent_cluster(S, kern, dim3(unsigned(tiles) * S), dim3(NTHREADS), SMEM_BYTES, stream, tm_x, tm_w, p));
+  count_launch();
+  return ALG_OK;
 }
 
 }  // namespace
 
-// The residual GEMM's tile is 128 x 256 unless 128 x 128 tiles spread better over the SMs (few rows: a
+// The residual GEMM's tiles are 128 x 256 unless 128 x 128 ones spread better over the SMs (few rows: a short prompt, or a
 // rank's share of a batch split over many GPUs).  Cost model: rounds of tiles per CTA times the time of
 // one tile.  A narrow tile takes a little more than half of a wide one while its rows come from L2; from HBM about
 // two thirds, its operands being 32 KB per 256 cycles of products (K = 2688, N = 1024: 8192 rows, 44 MB, 34.0 us narrow
@@ -637,7 +790,8 @@ int proj_resid_tile_width(int M, int N) {
   return cost_narrow < cost_wide ? 128 : 256;
 }
 
-int launch_proj(const ProjParams& p, const void* x, const void* w, int epi, cudaStream_t stream) {
+int launch_proj(const ProjParams& params, const void* x, const void* w, int epi, cudaStream_t stream) {
+  ProjParams p = params;
   if (p.M == 0) return ALG_OK;
   CUtensorMap tm_x, tm_w;
   {
@@ -646,18 +800,34 @@ int launch_proj(const ProjParams& p, const void* x, const void* w, int epi, cuda
     const uint32_t box[2] = {BK, BM};
     if (int rc = make_tmap_bf16(&tm_x, x, 2, dims, strides, box, true)) return rc;
   }
-  const int bn = epi == EPI_RESID ? proj_resid_tile_width(p.M, p.N) : BN_MAX;
+  // QKV (head_dim 64) and GLU: narrow tiles only where they are one round - their epilogues weigh more than the residual's
+  // (GLU 1024 x 1024 x 2688, 2 wide rounds or 3 narrow ones: 16.5 and 20.0 us; QKV 613 x 768, one of either: 10.0 and 7.9)
+  int bn = BN_MAX;
+  if (epi == EPI_RESID) bn = proj_resid_tile_width(p.M, p.N);
+  else if ((epi == EPI_GLU || (epi == EPI_QKV && p.D == 64)) && ((p.M + BM - 1) / BM) * ((p.N + 127) / 128) <= sm_count()) bn = 128;
   const int cg = bn == BN_MAX ? pair_size((p.M + BM - 1) / BM, (p.N + bn - 1) / bn, p.K / BK) : 1;
   {
     const uint64_t dims[2] = {uint64_t(p.K), uint64_t(p.N)};
     const uint64_t strides[1] = {uint64_t(p.K)};
-    const uint32_t box[2] = {BK, uint32_t(bn / cg)};
+    const uint32_t box[2] = {BK, epi == EPI_GLU && bn == 128 ? 64u : uint32_t(bn / cg)};
     if (int rc = make_tmap_bf16(&tm_w, w, 2, dims, strides, box, true)) return rc;
   }
   const int places = sm_count() / cg;
   const int tiles = ((p.M + cg * BM - 1) / (cg * BM)) * ((p.N + bn - 1) / bn);
+  // one round: the next kernel's CTAs set up on the SMs left free (hidden states of the 125M model, 613 tokens: 653 -> 604 us;
+  // with more rounds they would sit beside running ones)
+  p.announce = tiles <= places;
+  if (epi == EPI_RESID && bn == 128) {
+    // K over four CTAs from 16 ring steps on, over two from 32, where the chip has room (613 rows, K = 2048: 11.6 us whole, 10.1
+    // over two, 8.3 over four; 64 rows 11.3 and 7.5; 1024 x 2688 x 1024 14.3 and 12.0 over two).  Shorter K do not pay for
+    // the exchange (613 x 768 x 768, 12 steps: 6.7 whole, 7.7 and 6.9; 1024 x 1024 x 1024, 16 steps: 7.9 and 8.5 over two).
+    const int steps = p.K / BK;
+    if (steps >= 16 && tiles * 4 <= places) return launch_split<4>(tm_x, tm_w, p, tiles, stream);
+    if (steps >= 32 && tiles * 2 <= places) return launch_split<2>(tm_x, tm_w, p, tiles, stream);
+  }
   const int grid = (tiles < places ? tiles : places) * cg;
-  return cg == 2 ? launch_cg<2>(tm_x, tm_w, p, epi, bn, grid, stream) : launch_cg<1>(tm_x, tm_w, p, epi, bn, grid, stream);
+  if (cg == 2) return launch_tile<256, 2>(tm_x, tm_w, p, epi, grid, stream);
+  return bn == 128 ? launch_tile<128, 1>(tm_x, tm_w, p, epi, grid, stream) : launch_tile<256, 1>(tm_x, tm_w, p, epi, grid, stream);
 }
 
 }  // namespace alg

@@ -162,6 +162,17 @@ __device__ __forceinline__ uint32_t leader_smem(const void* p) {
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
+// Four floats at `addr`, an address in this CTA's shared memory, of the CTA of rank `rank` in the cluster.
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr, uint32_t rank) {
+  float4 v;
+  asm volatile(
+      "{\n"
+      ".reg .u32 a;\n"
+      "mapa.shared::cluster.u32 a, %4, %5;\n"
+      "ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [a];\n"
+      "}\n" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr), "r"(rank) : "memory");
+  return v;
+}
 // Tiled load into this CTA's shared memory whose bytes are counted on the leader's barrier.
 __device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* m, uint32_t leader_bar, int x, int y) {
   asm volatile(
