@@ -247,7 +247,7 @@ head_tc_kernel(const __grid_constant__ CUtensorMap tm_h, const __grid_constant__
         tc_fence_before();
         __syncwarp();
         if (lane == 0) {                                 // this warp is done reading the buffer
-          if (CG == 2) mbar_arrive_cluster(leader_smem(&ctl->tempty[buf]));
+          if (CG == 2) mbar_arrive_remote(leader_smem(&ctl->tempty[buf]));
           else mbar_arrive(&ctl->tempty[buf]);
         }
       }

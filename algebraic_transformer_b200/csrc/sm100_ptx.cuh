@@ -159,8 +159,12 @@ __device__ __forceinline__ uint32_t leader_smem(const void* p) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"(smem_u32(p)));
   return a;
 }
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+// An arrival on another CTA's barrier that publishes nothing but this thread's progress (tensor memory read, under
+// tcgen05.fence::before_thread_sync).  CTA scope on purpose: released at cluster scope it would first wait for the
+// thread's global stores to be performed, a trip to L2 per tile (it made membar the second largest stall of the
+// projections' epilogues).
+__device__ __forceinline__ void mbar_arrive_remote(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 // Four floats at `addr`, an address in this CTA's shared memory, of the CTA of rank `rank` in the cluster.
 __device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr, uint32_t rank) {
