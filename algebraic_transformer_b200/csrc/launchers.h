@@ -14,7 +14,7 @@ namespace alg {
 // single CTA, which has to be won back.  `row_blocks` 128-row blocks times `columns` tiles, or runs of tiles, of `steps`
 // ring steps beside each other.  Measured, single -> pairs: QKV 8192 x 768 (48 steps) 26.9 -> 28.6 us, 16384 x 1536 (768)
 // 177 -> 158; GLU 8192 x 768 (84) 41.6 -> 40.5, 16384 x 1536 (1392) 310 -> 272; down 16384 x 2048 x 768 (96) 46.2 -> 43.4,
-// out 16384 x 768 x 768 (36) 20.6 -> 22.8; head 8192 x 768 x 50304 441 -> 414, its gradient kernel 751 -> 659, head of 613
+// out 16384 x 768 x 768 (36) 20.6 -> 22.8; head 8192 x 768 x 50304 441 -> 392, its gradient kernel 751 -> 586, head of 613
 // rows (5 blocks: a sixth of the pairs' work is padding) 45.5 -> 48.4.
 inline int pair_size(int row_blocks, int columns, int steps) {
   const int64_t sms = sm_count(), pairs = sms / 2;

@@ -196,6 +196,9 @@ __device__ __forceinline__ void dz_cols(const ProjParams& p, uint32_t taddr, con
       tmem_ld_32x32(taddr + u * 64 + c * 32, r);
       tmem_ld_wait();
       const int cbase = col0 + u * 64 + c * 32;
+      // Every column is evaluated as one that is not the target; the target's pair is done again where it lies among these
+      // columns, which few warps see (a comparison and a selection per column were a fifth of the arithmetic).
+      const unsigned at = unsigned(tgt - cbase);
       if (p.head_kind == ALG_HEAD_CE) {
         // softmax cross-entropy: dz = (g / N) (exp(z - lse) - y), `inv_l` carries the row's logsumexp
         // (src/algebraic/kernels/fused_head.py:134-135)
@@ -205,8 +208,16 @@ __device__ __forceinline__ void dz_cols(const ProjParams& p, uint32_t taddr, con
         for (int i = 0; i < 32; i += 2) {
           const float p0 = exp2_approx(fmaf(__uint_as_float(r[i]), LOG2E, off));
           const float p1 = exp2_approx(fmaf(__uint_as_float(r[i + 1]), LOG2E, off));
-          pk[c * 16 + (i >> 1)] = pack_bf16(a_i * (p0 - ((cbase + i == tgt) ? 1.f : 0.f)),
-                                            a_i * (p1 - ((cbase + i + 1 == tgt) ? 1.f : 0.f)));
+          pk[c * 16 + (i >> 1)] = pack_bf16(a_i * p0, a_i * p1);
+        }
+        if (at < 32u) {
+#pragma unroll
+          for (int i = 0; i < 32; i += 2) {
+            if ((at | 1u) != unsigned(i | 1)) continue;
+            const float p0 = exp2_approx(fmaf(__uint_as_float(r[i]), LOG2E, off));
+            const float p1 = exp2_approx(fmaf(__uint_as_float(r[i + 1]), LOG2E, off));
+            pk[c * 16 + (i >> 1)] = pack_bf16(a_i * (p0 - (at == unsigned(i) ? 1.f : 0.f)), a_i * (p1 - (at == unsigned(i + 1) ? 1.f : 0.f)));
+          }
         }
         continue;
       }
@@ -233,9 +244,17 @@ __device__ __forceinline__ void dz_cols(const ProjParams& p, uint32_t taddr, con
       }
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
-        const float2 negy = make_float2((cbase + 2 * i == tgt) ? -1.f : 0.f, (cbase + 2 * i + 1 == tgt) ? -1.f : 0.f);
-        const float2 d = __fmul2_rn(sl[i], __ffma2_rn(w[i], il2, negy));
+        const float2 d = __fmul2_rn(sl[i], __fmul2_rn(w[i], il2));
         pk[c * 16 + i] = pack_bf16(d.x, d.y);
+      }
+      if (at < 32u) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          if ((at >> 1) != unsigned(i)) continue;
+          const float2 negy = make_float2(at == unsigned(2 * i) ? -1.f : 0.f, at == unsigned(2 * i + 1) ? -1.f : 0.f);
+          const float2 d = __fmul2_rn(sl[i], __ffma2_rn(w[i], il2, negy));
+          pk[c * 16 + i] = pack_bf16(d.x, d.y);
+        }
       }
     }
     const int first = col0 + u * 64;
