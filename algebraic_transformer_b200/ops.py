@@ -506,8 +506,8 @@ def flash_attention_backward(q, k, v, o, d_o, stat, stat_kind, sink_logit=None, 
     forward's inputs, its output `o`, the incoming gradient `d_o` and the saved `(stat, stat_kind)`
     (the custom VJP of the reference, src/algebraic/kernels/flash.py:333-727).  bf16 tensors,
     (B,H,T,D) with D contiguous; `dsink` is None without a sink.  `impl`: "auto" runs the tcgen05
-    kernels when the call is causal self-attention and the mma.sync
-    kernels otherwise; "mma" always runs the latter."""
+    kernels when the call is causal self-attention and the mma.sync kernels otherwise; "mma" always runs
+    the latter."""
     if impl not in ("auto", "mma"):
         raise ValueError('impl must be "auto" or "mma"')
     _require_cuda(q, k, v, o, d_o, stat, stat_kind)

@@ -6,8 +6,9 @@ RMS(embed_gain) -> L x [RMS -> QKV GEMMs -> QK-norm + Cayley rotation + asinh at
 (one library call) -> out-projection + residual -> RMS -> gate/up GEMMs -> gate * ALU(up)
 -> down GEMM + residual] -> final RMS -> fused Alg-CE head over all positions.
 Every stage is a kernel of this package, and all blocks are issued by one native call
-(`fused_norm=False`, or shapes the fused projections do not take: library GEMMs for the projections).  Projections are consumed in place as strided (B,H,T,D) views and the
-attention output is written straight into (B,T,H*D) layout, so no transposes are copied.
+(`fused_norm=False`, or shapes the fused projections do not take: library GEMMs).  Projections are
+consumed in place as strided (B,H,T,D) views and the attention output is written straight into
+(B,T,H*D) layout, so no transposes are copied.
 
 Multi-GPU (one process per GPU): the batch is split over ranks (weights replicated, no
 communication in the body), the final hidden states are all-gathered, and the head runs
