@@ -10,15 +10,20 @@
 // What bounded the loop before was instruction issue, not HBM: eight lanes shared a key's products
 // and all eight evaluated its weight, 200 instructions of a warp for 8 keys of head_dim 64, so caches of
 // a few thousand keys streamed at 3.9 TB/s.  Now both products run on the tensor cores as
-// mma.sync.m16n8k16 and a warp spends about 130 instructions on 32 keys:
+// mma.sync.m16n8k16, and a warp spends on 32 keys what it spent on 8:
 //   scores   A = q in every one of the first eight rows, B = K rows as they lie in shared memory
 //            (bf16 x bf16 is exact in fp32, as the scalar products were); every row of the result holds the
 //            32 scores, lane (r, i) = (lane / 4, lane % 4) those of keys 2 i, 2 i + 1 of each block of eight;
 //   weights  lane (r, i) evaluates the one key 8 (r / 2) + 2 i + r % 2;
-//   output   A row 0 = bf16(w), A row 1 = bf16(w - row 0): the pair carries w to 2^-17, and their sum is what
-//            the accumulator rows 0 and 1 add up to; B = V rows through ldmatrix.trans.  The remaining rows
-//            of A are free and ignored.  The normaliser adds the fp32 weights.
-// Single-row products leave 14 of the 16 rows idle, which costs nothing: the tensor pipe is at a few percent.
+//   output   A rows 0, 1, 2 = the three bf16 that add up to the fp32 weight, 8 bits of it each, so that the
+//            accumulator rows 0, 1 and 2 add up to what fp32 weights would give; B = V rows through ldmatrix.trans.
+//            The remaining rows of A are ignored.  The normaliser adds the fp32 weights.
+//            (With two parts, 16 of the 24 bits, the error before the output's rounding was ten times that of fp32
+//            products: 1.1e-6 against 1.1e-7 rms of the terms' size with two keys and n = 2, 1.16e-7 now; of
+//            5.2 million outputs over 64 to 60000 keys 8935 were not the nearest bf16, 4790 with fp32 products, 4871 now.  The
+//            third part costs nothing at head_dim 64 and on single CTAs, 2 to 4 % where two CTAs of head_dim 128 share an
+//            SM: 16 x 12 x 3000 x 128 57.9 -> 59.0 us, 32 x 24 x 300 x 128 33.0 -> 34.5.)
+// Single-row products leave 13 of the 16 rows idle, which costs nothing: the tensor pipe is at a few percent.
 //
 // The warp states are merged once at the end with the exact rescale (rho(m_a) rho(-m))^n.  A CTA
 // that holds a whole head writes the output row; otherwise it writes its (acc, m, l) state and the split
@@ -28,7 +33,7 @@
 // zero arrivals).  All mbarrier waits are bounded.
 //
 // Measured (CUDA graph, before -> now): 16 x 16 heads x 1900 keys x 64 31.7 -> 21.7 us = 5.7 TB/s, 1 x 16 x 32768 x 128
-// 55.5 -> 47.5 = 5.65 TB/s, 16 x 12 x 3000 x 128 73 -> 59, 32 x 24 x 64 x 64 15.4 -> 9.4, 1 x 12 x 333 x 64 9.7 -> 8.2, of which
+// 55.5 -> 47.5 = 5.65 TB/s, 16 x 12 x 3000 x 128 73 -> 59, 32 x 24 x 64 x 64 15.4 -> 9.6, 1 x 12 x 333 x 64 9.7 -> 8.2, of which
 // about 8 is a launch, the first tile's way and the merge.
 #include "common.cuh"
 #include "launchers.h"
@@ -174,7 +179,7 @@ decode_partial_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
     const uint32_t* q32 = reinterpret_cast<const uint32_t*>(static_cast<const __nv_bfloat16*>(p.q) + (int64_t(b) * p.H + h) * D);
 #pragma unroll
     for (int ks = 0; ks < D / 16; ++ks) { qa[ks][0] = q32[ks * 8 + i]; qa[ks][1] = q32[ks * 8 + 4 + i]; }
-    float acc[D / 8][2];                        // rows 0 and 1: high and low halves of the weights times V
+    float acc[D / 8][2];                        // rows 0, 1, 2: the three parts of the weights times V
 #pragma unroll
     for (int c = 0; c < D / 8; ++c) acc[c][0] = acc[c][1] = 0.f;
     float m_ref = -1e30f, shift = 0.f, l_part = 0.f;
@@ -184,7 +189,8 @@ decode_partial_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
     const uint32_t v_row = uint32_t(((lane >> 3) & 1) * 8 + (lane & 7)) * 128, v_chunk = uint32_t(lane >> 4);   // + 16 keys, + 2
     const uint32_t swz = uint32_t(lane & 7);
     const int own = 8 * (r >> 1) + 2 * i + (r & 1);                                              // the key this lane evaluates
-    const uint32_t halves = r == 1 ? 0x7632u : 0x5410u;                                          // this row's half of a weight
+    const bool odd = (r & 1) != 0;
+    const uint32_t part = uint32_t(i) | (r == 0 ? 0u : r == 1 ? 4u : 8u);                        // the lane that has this row's part of a weight
     bool ok = true;
     for (int t = warp; t < ntiles; t += CWARPS) {
       const int stage = t % STAGES;
@@ -219,16 +225,21 @@ decode_partial_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
       }
       const float w = (x > -1e29f) ? pow2n_rt(rho_stable(x) * shift, p.log2n) : 0.f;
       l_part += w;
-      const float hi = __bfloat162float(__float2bfloat16_rn(w));
-      const uint32_t both = pack_bf16(w, w - hi);
+      // w = h + m + lo, three bf16 that carry all 24 bits of it.  Two neighbouring keys' lanes (even and odd row) exchange
+      // halves: the even one then has both keys' h, the odd one both m, either both lo, which also go to the
+      // lanes of the neighbouring block of eight keys.  One shuffle per block then serves rows 0, 1 and 2.
+      const float h = __bfloat162float(__float2bfloat16_rn(w)), m = __bfloat162float(__float2bfloat16_rn(w - h)), lo = w - h - m;
+      const uint32_t kept = pack_bf16(odd ? m : h, lo);
+      const uint32_t got = __shfl_xor_sync(0xffffffffu, pack_bf16(odd ? h : m, lo), 4);
+      const uint32_t lead = __byte_perm(kept, got, odd ? 0x1054u : 0x5410u);
+      const uint32_t rest = __shfl_xor_sync(0xffffffffu, __byte_perm(kept, got, odd ? 0x3276u : 0x7632u), 8);
 #pragma unroll
       for (int ks = 0; ks < 2; ++ks) {          // sixteen keys
         uint32_t wa[2];
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {           // keys 2 i, 2 i + 1 of block 2 ks + j: evaluated by rows 2 (2 ks + j), + 1
-          const uint32_t w0 = __shfl_sync(0xffffffffu, both, (2 * (2 * ks + j)) * 4 + i);
-          const uint32_t w1 = __shfl_sync(0xffffffffu, both, (2 * (2 * ks + j) + 1) * 4 + i);
-          wa[j] = __byte_perm(w0, w1, halves);
+        for (int j = 0; j < 2; ++j) {           // keys 2 i, 2 i + 1 of block 2 ks + j
+          const int block = 2 * ks + j;
+          wa[j] = __shfl_sync(0xffffffffu, (r >> 1) == block ? lead : rest, (block * 8) ^ int(part));
         }
 #pragma unroll
         for (int c = 0; c < D / 8; c += 2) {    // sixteen columns of V a load
@@ -241,7 +252,7 @@ decode_partial_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
       __syncwarp();
       if (lane == 0) mbar_arrive(&ctl->empty[stage]);      // this warp is done with the stage
     }
-    // ---- this warp's state: rows 0 and 1 together, then merge the warps
+    // ---- this warp's state: rows 0, 1 and 2 together, then merge the warps
     __syncwarp();
     l_part = warp_sum(l_part);
     consumer_sync<C::CONSUMERS>();                          // ring no longer read: reuse it as scratch
@@ -250,9 +261,9 @@ decode_partial_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
     for (int c = 0; c < D / 8; ++c) {
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        const float lo = __shfl_down_sync(0xffffffffu, acc[c][e], 4);
-        // an infinite V meets a zero low half as NaN: the high half has the answer then
-        if (r == 0) s_acc[warp * D + c * 8 + 2 * i + e] = isinf(acc[c][e]) ? acc[c][e] : acc[c][e] + lo;
+        const float mid = __shfl_down_sync(0xffffffffu, acc[c][e], 4), low = __shfl_down_sync(0xffffffffu, acc[c][e], 8);
+        // an infinite V meets a zero part of a weight as NaN: the leading part has the answer then
+        if (r == 0) s_acc[warp * D + c * 8 + 2 * i + e] = isinf(acc[c][e]) ? acc[c][e] : acc[c][e] + (mid + low);
       }
     }
     if (lane == 0) { ctl->m[warp] = m_ref; ctl->l[warp] = l_part; if (!ok) ctl->tile_ok = 0; }
@@ -344,7 +355,9 @@ int launch_d(const DecodeParams& p, cudaStream_t stream) {
 // beside each other; what decides is how full the last round of CTAs is.  Heads up to the SM count are split to fill
 // one round, and heads that take an odd number of rounds of single CTAs would waste half a round in pairs: one.
 // Measured, two -> one: 1 x 16 x 32768 57 -> 47.5 us, 7 x 6 x 5000 30.2 -> 24.0, 16 x 24 x 1000 (3 rounds) 47.9 -> 39.9;
-// 16 x 12 x 500 (2 rounds) 13.6 -> 15.0, 32 x 24 x 300 (6 rounds) 33.6 -> 41.2.
+// 16 x 12 x 500 (2 rounds) 13.6 -> 15.0, 32 x 24 x 300 (6 rounds) 33.6 -> 41.2.  75 to 147 heads in single CTAs are one
+// unsplit CTA each and leave SMs idle, which loses nothing to speak of: the CTAs' rings together already
+// draw what HBM gives (4 x 24 x 8192 59.4 us = 6.8 TB/s on 96 SMs, 5 x 16 x 8192 56.8 us = 5.9 TB/s on 80).
 static int ctas_per_sm(int D, int B, int H) {
   const int sms = sm_count();
   return D == 128 && ((int64_t(B) * H + sms - 1) / sms) % 2 == 1 ? 1 : 2;

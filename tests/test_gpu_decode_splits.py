@@ -1,6 +1,8 @@
 """Decode at the sizes where its grid rule turns or a ring slot, a tile or a split is not full: one key, one tile and one
 key more, one CTA per head and several, one and two CTAs per SM, more heads than CTAs fit."""
 
+import math
+
 import pytest
 import torch
 
@@ -45,3 +47,29 @@ def test_decode_extremes(D):
     args[1][0, 0, 5] = args[0][0, 0, 0]                            # a key with weight
     got = A.decode_attention(*args, n=16, c=8.0).float()
     assert got[0, 0, 0, 3] == float("inf") and torch.isfinite(got[0, 1]).all() and torch.isfinite(got[0, 0, 0, :3]).all()
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_decode_weights_keep_their_bits(D):
+    """Two keys whose contributions cancel to about 2^-14: the output's rounding is far below the error of the weights.
+
+    n = 2, so that nothing multiplies the error of a weight up: one score (2^-22 of it), one rho on either side of the shift
+    (2^-22 each, approximate square root), a power of two and fp32 sums: below 2^-20 of the terms' size.  Weights cut to 16
+    bits are off by up to 2^-18."""
+    B, H, c = 4, 64, 8.0
+    q, k = (randn((B, H, n, D), 61 + i, torch.bfloat16) for i, n in enumerate((1, 2)))
+    x = (k.double() @ q.double().transpose(-1, -2))[..., 0] / (math.sqrt(D) * c)
+    w = (x + torch.sqrt(1 + x * x)) ** 2
+    ratio = w[..., :1] / w[..., 1:]
+    v0 = torch.arange(128, 256).double() / 128                     # every mantissa of a bf16
+    e = 2.0 ** torch.floor(torch.log2(ratio * v0))
+    v1 = (ratio * v0 / e * 128).round() / 128 * e                  # the bf16 nearest to what would cancel it
+    best = ((ratio * v0 - v1).abs() / v1).argsort(-1)[..., :D]
+    v = torch.stack([v0[best], -torch.gather(v1, -1, best)], 2).bfloat16()
+    got = A.decode_attention(q.to(DEV), k.to(DEV), v.to(DEV), n=2, c=c).cpu().double()[:, :, 0]
+    terms = w[..., None] * v.double() / w.sum(-1)[..., None, None]
+    want, size = terms.sum(2), terms.abs().sum(2)
+    rounding = want.abs() * 2.0 ** -8                              # a bf16 next to the nearest one
+    seen = rounding < 2.0 ** -22 * size                            # where the output shows the weights' error
+    assert int(seen.sum()) > 1000
+    assert float(((got - want).abs() / size)[seen].max()) < 2.0 ** -20 + 2.0 ** -22
