@@ -68,7 +68,7 @@ template <int D, int BS, int CTAS> struct Cfg {
   static constexpr int NG = BS / 32;                            // column groups of the element-wise stage
   static constexpr int EW_WARPS = 4 * NG, NTHREADS = 64 + 32 * EW_WARPS;
   static constexpr int RING_OFF = 2 * RES_BYTES;
-  static constexpr int VEC_OFF = RING_OFF + NS * 2 * STR_BYTES; // MODE 1: per ring slot BS weight factors, BS negated deltas
+  static constexpr int VEC_OFF = RING_OFF + NS * 2 * STR_BYTES; // MODE 1: per ring slot BS statistics, BS negated deltas
   static constexpr int CTL_OFF = VEC_OFF + NS * 2 * BS * 4;
   static constexpr uint32_t TMEM_COLS = 512 / CTAS;
   static constexpr uint32_t S_COL = 0, DP_COL = BS, ACC0_COL = 2 * BS, ACC1_COL = 2 * BS + D;
@@ -92,9 +92,11 @@ template <class C> constexpr size_t smem_bytes() { return size_t(C::CTL_OFF) + s
 // p / sqrt(1 + x^2) that phase 2 multiplies (dP - delta) by.  Packed fp32 pairs throughout.
 //
 // Unshifted statistic (1 / l): with y the raw score, s = 1 / (sqrt(D) c) and kappa = 1 / s^2,
-//   p = rho(x)^n / l = (a (y + sqrt(kappa + y^2)))^n,  a = s l^(-1/n),
-// and 1 / sqrt(1 + x^2) = rsqrt(kappa + y^2) / s, so neither the score scale nor the statistic costs a
-// multiplication of its own; the constant 1 / s joins the factors n s that the epilogue applies.
+//   p = (s (y + sqrt(kappa + y^2)))^n / l  and  1 / sqrt(1 + x^2) = rsqrt(kappa + y^2) / s;
+// the constant 1 / s joins the factors n s that the epilogue applies.  The statistic multiplies the finished power: as
+// s l^(-1/n) ahead of it, one multiplication less, its own rounding came out of the power n times as large, and the
+// kernel was hardly faster for it ((16,12,1024,64) 182.0 us against 180.9, (8,16,2048,64) 383 and 384, (1,16,8192,64) 608
+// against 622, (2,16,1837,128) 143 and 142).
 // Shifted statistic (rho(-m) l^(-1/n)): p = (rho(x) a)^n with the cancellation-free rho and a = the statistic.
 // `a` comes by row (MODE 0: a2[0]) or by column (MODE 1: a2[0..7]).
 template <bool SHIFTED, bool BY_COLUMN, int LOG2N, bool MASK>
@@ -115,7 +117,7 @@ __device__ __forceinline__ void weights16(const uint32_t* s, float2* slope, uint
       slope[i] = make_float2(rsqrt_approx(rad.x), rsqrt_approx(rad.y));
       t[i] = __ffma2_rn(rad, slope[i], y);
     }
-    t[i] = __fmul2_rn(t[i], BY_COLUMN ? a2[i] : a2[0]);
+    t[i] = __fmul2_rn(t[i], !SHIFTED ? sc : BY_COLUMN ? a2[i] : a2[0]);
   }
   // the power as passes over the eight pairs, so that every pass has independent multiplications
   if (LOG2N > 0) {
@@ -127,6 +129,10 @@ __device__ __forceinline__ void weights16(const uint32_t* s, float2* slope, uint
     for (int it = 0; it < log2n; ++it)
 #pragma unroll
       for (int i = 0; i < 8; ++i) t[i] = __fmul2_rn(t[i], t[i]);
+  }
+  if (!SHIFTED) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) t[i] = __fmul2_rn(t[i], BY_COLUMN ? a2[i] : a2[0]);
   }
   if (MASK) {   // causal, key <= query: rows are keys where the factors come by column, else queries
 #pragma unroll
@@ -143,7 +149,7 @@ __device__ __forceinline__ void weights16(const uint32_t* s, float2* slope, uint
   }
 }
 
-// Phase 1 on this thread's 32 scores at tensor-memory address s_t; `vec`: the columns' factors in shared memory
+// Phase 1 on this thread's 32 scores at tensor-memory address s_t; `vec`: the columns' statistics in shared memory
 // (MODE 1).  MODE 1 leaves the packed weights over the columns read.
 template <int MODE, bool SHIFTED, int LOG2N, bool MASK>
 __device__ __forceinline__ void phase1(uint32_t s_t, float2* slope, const float* vec, float2 a_row, float scale, float kappa,
@@ -170,13 +176,6 @@ __device__ __forceinline__ void phase1(uint32_t s_t, float2* slope, const float*
     weights16<SHIFTED, MODE == 1, LOG2N, MASK>(c == 0 ? s0 : s1, slope + 8 * c, pw, a2, scale, kappa, log2n, row, col0 + c * 16);
     if (MODE == 1) tmem_st_32x8(s_t + c * 8, pw);
   }
-}
-
-// What a weight needs of a query's saved statistic: a of weights16.
-__device__ __forceinline__ float weight_factor(float stat, bool shifted, float scale, int log2n) {
-  if (shifted) return stat;
-  for (int i = 0; i < log2n; ++i) stat = sqrtf(stat);
-  return stat * scale;
 }
 
 template <class C, int D, int BS, int MODE>
@@ -239,7 +238,7 @@ __device__ __forceinline__ void bwd_block(unsigned char* smem, Control* ctl, con
         float* vec = reinterpret_cast<float*>(smem + C::VEC_OFF) + slot * 2 * BS;
 #pragma unroll
         for (int i = 0; i < VPL; ++i) {
-          vec[i * 32 + lane] = weight_factor(st[i], shifted, p.scale, p.log2n);
+          vec[i * 32 + lane] = st[i];
           vec[BS + i * 32 + lane] = -dl[i];
         }
         __syncwarp();
@@ -325,7 +324,7 @@ __device__ __forceinline__ void bwd_block(unsigned char* smem, Control* ctl, con
     const float kappa = 1.0f / (p.scale * p.scale);
     float2 a_row = make_float2(0.f, 0.f), delta_row = make_float2(0.f, 0.f);
     if (MODE == 0 && row < p.Tq) {
-      const float a = weight_factor(p.stat[bh * p.Tq + row], shifted, p.scale, p.log2n), d = -p.delta[bh * p.Tq + row];
+      const float a = p.stat[bh * p.Tq + row], d = -p.delta[bh * p.Tq + row];
       a_row = make_float2(a, a);
       delta_row = make_float2(d, d);
     }
@@ -436,8 +435,8 @@ __device__ __forceinline__ void bwd_block(unsigned char* smem, Control* ctl, con
     // dsink: -sum_i delta_i p_sink,i n / (c sqrt(1 + (b/c)^2)), one atomic per warp of the first column group
     if (MODE == 0 && p.sink != nullptr && p.dsink != nullptr && group == 0) {
       const float bs = p.sink[h] * p.inv_c;
-      const float a = shifted ? a_row.x : a_row.x / p.scale;
-      float part = delta_row.x * pow2n_rt(rho_stable(bs) * a, p.log2n) * p.n_f * p.inv_c * rsqrtf(fmaf(bs, bs, 1.0f));
+      const float ps = shifted ? pow2n_rt(rho_stable(bs) * a_row.x, p.log2n) : pow2n_rt(rho_stable(bs), p.log2n) * a_row.x;
+      float part = delta_row.x * ps * p.n_f * p.inv_c * rsqrtf(fmaf(bs, bs, 1.0f));
       part = warp_sum(part);
       if (lane == 0) atomicAdd(p.dsink + h, part);
     }

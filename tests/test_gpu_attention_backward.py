@@ -78,3 +78,19 @@ def test_backward_stores_nothing_past_the_end(D):
     for got, w in zip(outs, want):
         assert torch.equal(got[:B * H * T * D].view(B, H, T, D), w)
         assert (got[B * H * T * D:] == 7.0).all()
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_statistic_is_not_amplified(D):
+    """The sink's gradient, the one fp32 output, for single rows: with a zero sink and one element of `d_o` it is a product of
+    exact numbers, n, 1 / c and the saved 1 / l: five roundings.  l^(-1/n) raised to n again would be off by up to 16."""
+    H, n, c = 512, 16, 8.0
+    q, k, v = (randn((1, H, 1, D), 71 + i, torch.bfloat16).to(DEV) for i in range(3))
+    sink = torch.zeros(H, device=DEV)
+    o, stat, which = A.flash_attention(q, k, v, sink, kind="asinh", n=n, c=c, block=1, range_guard=True, return_stat=True)
+    d_o = torch.zeros_like(o)
+    d_o[..., 3] = 1.0
+    assert int(which) == 1                                         # the unshifted form
+    dsink = A.flash_attention_backward(q, k, v, o, d_o, stat, which, sink, n=n, c=c)[3]
+    want = -(o[0, :, 0, 3].double() * stat[0, :, 0].double() * n / c)
+    assert float(((dsink.double() - want) / want).abs().max()) < 5 * 2.0 ** -24
