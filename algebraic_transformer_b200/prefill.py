@@ -144,9 +144,6 @@ class Prefill:
         self.p = cast_params(params, self.device, self.fused_proj, self.norm_in_weights)
         self.cos, self.sin = ops.cayley_table_geometric(cfg.head_dim, seq_len, cfg.rope_base, device=self.device)
         self.cos_lp, self.sin_lp = self.cos.bfloat16().contiguous(), self.sin.bfloat16().contiguous()
-        # one record of the range guard's maxima per layer: all zeroed by one fill at the start of a step,
-        # so that no memset sits between two kernels of the step
-        self.guard_words = torch.zeros((cfg.n_layers, 4), dtype=torch.int32, device=self.device)
 
     def hidden(self, tokens: torch.Tensor) -> torch.Tensor:
         """Final normalised hidden states (B, T, d) in bf16 (model.forward_hidden, model.py:196-208)."""
@@ -155,11 +152,13 @@ class Prefill:
         d, H, D, f = cfg.d_model, cfg.n_heads, cfg.head_dim, cfg.d_ff
         x = ops.rms_norm(p["embed"][tokens].contiguous(), p["embed_gain"], cfg.eps).view(B * T, d)
         if self.fused_proj:
-            self.guard_words.zero_()
+            # one record of the range guard's maxima per layer: all zeroed by one fill at the start of a step,
+            # so that no memset sits between two kernels of the step; a call's own, since calls on two streams overlap
+            guard_words = torch.zeros((cfg.n_layers, 4), dtype=torch.int32, device=self.device)
         if self.norm_in_weights:
             # the norms as row scales inside the projections: five launches a block, all issued by one native call
             return ops.prefill_blocks(x, p["w_qkv_t"], p["w_o_t"], p["w_gu_t"], p["w_d_t"], p["q_gain"], p["k_gain"],
-                                      p["sink"], p["final_gain"], self.cos_lp, self.sin_lp, self.guard_words, batch=B,
+                                      p["sink"], p["final_gain"], self.cos_lp, self.sin_lp, guard_words, batch=B,
                                       n_heads=H, eps=cfg.eps, alu_beta=cfg.alu_beta, attn_n=cfg.attn_n, attn_c=cfg.attn_c,
                                       impl=self.impl).view(B, T, d)
         attn_out = torch.empty((B, T, H, D), dtype=torch.bfloat16, device=self.device)
@@ -167,11 +166,11 @@ class Prefill:
             h = ops.rms_norm(x, p["ln1"][layer], cfg.eps)
             if self.fused_proj:
                 qkv = ops.qkv_projection(h, p["w_qkv_t"][layer], H, T, self.cos_lp, self.sin_lp, p["q_gain"][layer],
-                                         p["k_gain"][layer], cfg.eps, cfg.attn_c, self.guard_words[layer],
+                                         p["k_gain"][layer], cfg.eps, cfg.attn_c, guard_words[layer],
                                          guard_is_zero=True).view(B, T, 3, H, D)
                 q, k, v = (qkv[:, :, i].transpose(1, 2) for i in range(3))      # (B,H,T,D) views
                 ops.flash_attention(q, k, v, p["sink"][layer], kind="asinh", n=cfg.attn_n, c=cfg.attn_c, block=T,
-                                    range_guard=True, impl=self.impl, guard_words=self.guard_words[layer],
+                                    range_guard=True, impl=self.impl, guard_words=guard_words[layer],
                                     out=attn_out.transpose(1, 2))
                 x = torch.addmm(x, attn_out.view(B * T, d), p["w_o"][layer])
                 h2 = ops.rms_norm(x, p["ln2"][layer], cfg.eps)
