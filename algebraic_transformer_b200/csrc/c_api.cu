@@ -3,6 +3,7 @@
 // synchronises: every call only enqueues work on the caller's stream.
 #include <math.h>
 #include <atomic>
+#include <chrono>
 #include <mutex>
 #include <stdarg.h>
 #include <stdio.h>
@@ -541,6 +542,14 @@ size_t alg_decode_workspace_bytes(const alg_decode_args* a) {
   return align256(size_t(a->B) * a->H * decode_splits(a->D, a->B, a->H, a->Tk) * (a->D + 2) * sizeof(float)) + size_t(a->B) * a->H * 8;
 }
 
+static unsigned long long call_numbers_from() {
+  static int here;                                      // an address that differs from process to process, like the time
+  unsigned long long x = static_cast<unsigned long long>(std::chrono::steady_clock::now().time_since_epoch().count()) ^
+                         (reinterpret_cast<uintptr_t>(&here) << 20);
+  for (int i = 0; i < 3; ++i) { x ^= x >> 31; x *= 0x9e3779b97f4a7c15ull; }
+  return x ^ (x >> 29);
+}
+
 int alg_attn_decode(const alg_decode_args* a, void* stream) {
   if (a == nullptr || a->q == nullptr || a->k == nullptr || a->v == nullptr || a->o == nullptr) {
     set_error("decode: null tensor argument");
@@ -572,8 +581,10 @@ int alg_attn_decode(const alg_decode_args* a, void* stream) {
   if (!aligned16(a->workspace)) { set_error("decode: workspace must be 16-byte aligned"); return ALG_ERR_INVALID; }
   p.arrivals = reinterpret_cast<unsigned long long*>(static_cast<unsigned char*>(a->workspace) +
                                                      align256(size_t(a->B) * a->H * p.splits * (a->D + 2) * sizeof(float)));
-  static std::atomic<unsigned long long> calls{0};
-  p.call = (calls.fetch_add(1) + 1) & ((1ull << 47) - 1);
+  // The workspace comes uninitialised: what lies there must not read as arrivals of this call.  Counted from one, the
+  // numbers would meet small integers and old words; counted from a place of the process's own they meet nothing likely.
+  static std::atomic<unsigned long long> calls{call_numbers_from()};
+  p.call = calls.fetch_add(1) & ((1ull << 47) - 1);
   return launch_decode(p, static_cast<cudaStream_t>(stream));
 }
 

@@ -2,6 +2,9 @@
 key more, one CTA per head and several, one and two CTAs per SM, more heads than CTAs fit."""
 
 import math
+import os
+import subprocess
+import sys
 
 import pytest
 import torch
@@ -73,3 +76,32 @@ def test_decode_weights_keep_their_bits(D):
     seen = rounding < 2.0 ** -22 * size                            # where the output shows the weights' error
     assert int(seen.sum()) > 1000
     assert float(((got - want).abs() / size)[seen].max()) < 2.0 ** -20 + 2.0 ** -22
+
+
+STALE_WORDS = """
+import torch
+from algebraic_transformer_b200 import _lib as L
+B, H, Tk, D = 1, 64, 1000, 64
+q, k, v = (torch.randn(B, H, n, D, device="cuda").bfloat16() for n in (1, Tk, Tk))
+o, want = torch.empty_like(q), None
+lib = L.load()
+a = L.DecodeArgs(q=q.data_ptr(), k=k.data_ptr(), v=v.data_ptr(), o=o.data_ptr(), B=B, H=H, Tk=Tk, D=D, n=16, c=8.0,
+                 k_stride=L.I64x3(*k.stride()[:3]), v_stride=L.I64x3(*v.stride()[:3]))
+size = lib.alg_decode_workspace_bytes(a)
+splits = (size - B * H * 8) // (B * H * (D + 2) * 4)
+assert splits > 1
+for _ in range(H):
+    ws = torch.full((size // 8,), -1, dtype=torch.int64, device="cuda")          # states: NaN
+    ws[-H:] = (torch.arange(H, device="cuda") + 1) * 65536 + splits - 1          # "all but one split of call 1, 2, ..."
+    a.workspace, a.workspace_bytes = ws.data_ptr(), size
+    assert lib.alg_attn_decode(a, torch.cuda.current_stream().cuda_stream) == 0
+    want = o.clone() if want is None else want
+    assert torch.isfinite(o).all() and torch.equal(o, want)
+"""
+
+
+def test_stale_arrival_words():
+    """A workspace that holds what the first calls of a process would leave, were their numbers counted from one."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", STALE_WORDS], cwd=root, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr
