@@ -134,6 +134,7 @@ SYMBOLS = {
     "alg_head_bwd_dz": (C.c_int, [C.POINTER(HeadBwdArgs), C.c_void_p]),
     "alg_decode_workspace_bytes": (C.c_size_t, [C.POINTER(DecodeArgs)]),
     "alg_attn_decode": (C.c_int, [C.POINTER(DecodeArgs), C.c_void_p]),
+    "alg_attn_decode_status": (C.c_int, [C.POINTER(DecodeArgs), C.c_void_p, C.c_void_p]),
     "alg_head_workspace_bytes": (C.c_size_t, [C.POINTER(HeadArgs)]),
     "alg_head_fwd": (C.c_int, [C.POINTER(HeadArgs), C.c_void_p]),
     "alg_head_fwd_static": (C.c_int, [C.POINTER(HeadArgs), C.c_void_p]),
@@ -153,6 +154,7 @@ SYMBOLS = {
     "alg_resid_proj_fwd": (C.c_int, [C.POINTER(ResidProjArgs), C.c_void_p]),
     "alg_resid_proj_ss_slots": (C.c_int, [C.c_int, C.c_int]),
     "alg_row_sumsq": (C.c_int, [C.c_void_p, C.c_int64, C.c_int, C.c_int64, C.c_void_p, C.c_void_p]),
+    "alg_selftest_decode_timeout": (C.c_int, [C.POINTER(DecodeArgs), C.c_int, C.c_ulonglong, C.c_void_p, C.c_void_p]),
     "alg_selftest_bounded_wait": (C.c_int, [C.c_void_p, C.c_ulonglong, C.c_void_p, C.c_void_p]),
     "alg_rms_norm_fwd":(C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int, C.c_float, C.c_void_p]),
     "alg_alu_glu_fwd": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int, C.c_int64, C.c_int64, C.c_float,

@@ -1,6 +1,7 @@
 // The C ABI declared in include/alg_b200.h: argument validation, workspace carving and
 // kernel selection.  Nothing here allocates device memory, creates streams or events, or
 // synchronises: every call only enqueues work on the caller's stream.
+#include <limits.h>
 #include <math.h>
 #include <atomic>
 #include <chrono>
@@ -550,7 +551,7 @@ static unsigned long long call_numbers_from() {
   return x ^ (x >> 29);
 }
 
-int alg_attn_decode(const alg_decode_args* a, void* stream) {
+static int decode_call(const alg_decode_args* a, int* status, unsigned long long wait_ns, int max_loads, void* stream) {
   if (a == nullptr || a->q == nullptr || a->k == nullptr || a->v == nullptr || a->o == nullptr) {
     set_error("decode: null tensor argument");
     return ALG_ERR_INVALID;
@@ -576,7 +577,9 @@ int alg_attn_decode(const alg_decode_args* a, void* stream) {
   }
   p.splits = decode_splits(a->D, a->B, a->H, a->Tk);
   p.keys_per_split = decode_keys_per_split(a->D, a->B, a->H, a->Tk);
-  p.status = nullptr;
+  p.status = status;
+  p.wait_ns = wait_ns;
+  p.max_loads = max_loads;
   p.part = static_cast<float*>(a->workspace);
   if (!aligned16(a->workspace)) { set_error("decode: workspace must be 16-byte aligned"); return ALG_ERR_INVALID; }
   p.arrivals = reinterpret_cast<unsigned long long*>(static_cast<unsigned char*>(a->workspace) +
@@ -586,6 +589,18 @@ int alg_attn_decode(const alg_decode_args* a, void* stream) {
   static std::atomic<unsigned long long> calls{call_numbers_from()};
   p.call = calls.fetch_add(1) & ((1ull << 47) - 1);
   return launch_decode(p, static_cast<cudaStream_t>(stream));
+}
+
+int alg_attn_decode(const alg_decode_args* a, void* stream) { return decode_call(a, nullptr, 1000000000ull, INT_MAX, stream); }
+
+int alg_attn_decode_status(const alg_decode_args* a, int* status, void* stream) {
+  return decode_call(a, status, 1000000000ull, INT_MAX, stream);
+}
+
+int alg_selftest_decode_timeout(const alg_decode_args* a, int max_loads, unsigned long long budget_ns, int* status, void* stream) {
+  if (status == nullptr || max_loads < 0) { set_error("selftest: status word and a tile count required"); return ALG_ERR_INVALID; }
+  if (budget_ns == 0 || budget_ns > 1000000000ull) { set_error("selftest: budget must be in (0, 1 s]"); return ALG_ERR_INVALID; }
+  return decode_call(a, status, budget_ns, max_loads, stream);
 }
 
 // Validation and parameter derivation shared by every head entry point (not exported).

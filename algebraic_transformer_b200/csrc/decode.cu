@@ -30,7 +30,8 @@
 // that finishes last for its (batch, head) merges the states, with the sink, and writes the output
 // row: one launch.  "Last" is decided by an arrival word per (batch, head) that carries the call's
 // number, so that nothing has to be zeroed between calls (a word left by another call counts as
-// zero arrivals).  All mbarrier waits are bounded.
+// zero arrivals).  All mbarrier waits are bounded; the row of a (batch, head) whose wait ran out is NaN, and the status
+// word, where there is one, says ALG_DEV_TIMEOUT.
 //
 // Measured (CUDA graph, before -> now): 16 x 16 heads x 1900 keys x 64 31.7 -> 21.7 us = 5.7 TB/s, 1 x 16 x 32768 x 128
 // 55.5 -> 47.5 = 5.65 TB/s, 16 x 12 x 3000 x 128 73 -> 59, 32 x 24 x 64 x 64 15.4 -> 9.6, 1 x 12 x 333 x 64 9.7 -> 8.2, of which
@@ -159,12 +160,13 @@ decode_partial_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
   if (threadIdx.x == C::CONSUMERS) { tma_prefetch_desc(&tm_k); tma_prefetch_desc(&tm_v); }
   __syncthreads();
   griddep_wait();                               // launched as a programmatic dependent of the kernel ahead in the stream
-  const BoundedWait bw{&ctl->abort_flag, 1000000000ull};
+  const BoundedWait bw{&ctl->abort_flag, p.wait_ns};
 
   if (warp == CWARPS) {                         // producer warp
     if (lane == 0) {
       uint32_t stage = 0, phase = 1;
-      for (int t = 0; t < ntiles; ++t) {
+      const int loads = min(ntiles, p.max_loads);
+      for (int t = 0; t < loads; ++t) {
         if (!bw.wait(&ctl->empty[stage], phase)) break;
         unsigned char* dst = smem + size_t(stage) * 2 * TILE_BYTES;
         mbar_arrive_expect_tx(&ctl->full[stage], 2 * TILE_BYTES);
@@ -269,7 +271,8 @@ decode_partial_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
     if (lane == 0) { ctl->m[warp] = m_ref; ctl->l[warp] = l_part; if (!ok) ctl->tile_ok = 0; }
     consumer_sync<C::CONSUMERS>();
     if (threadIdx.x < D) {
-      const bool fine = ctl->tile_ok != 0;
+      const bool fine = ctl->tile_ok != 0;                    // a wait that ran out leaves a row of NaN, not one of fewer keys
+      const float nan = __int_as_float(0x7fc00000);
       const bool sunk = p.splits == 1 && p.sink != nullptr;   // the sink joins here when this CTA has the whole head
       const float bs = sunk ? p.sink[h] * p.inv_c : -1e30f;
       float mm = bs;
@@ -285,13 +288,13 @@ decode_partial_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
         l = fmaf(f, ctl->l[wv], l);
       }
       if (p.splits == 1) {
-        reinterpret_cast<__nv_bfloat16*>(p.o)[(int64_t(b) * p.H + h) * D + threadIdx.x] = __float2bfloat16_rn(a / l);
+        reinterpret_cast<__nv_bfloat16*>(p.o)[(int64_t(b) * p.H + h) * D + threadIdx.x] = __float2bfloat16_rn(fine ? a / l : nan);
       } else {
         float* out = p.part + ((int64_t(b) * p.H + h) * p.splits + split) * (D + 2);
         out[threadIdx.x] = fine ? a : 0.f;
         if (threadIdx.x == 0) {
           out[D] = fine ? mm : -1e30f;
-          out[D + 1] = fine ? l : 0.f;
+          out[D + 1] = fine ? l : nan;                      // reaches the merged row as 0 * NaN
         }
         __threadfence();                                   // the state is visible before this split counts as arrived
       }

@@ -221,6 +221,8 @@ struct DecodeParams {
   float* part;             // (B*H, splits, D + 2) fp32 partials: acc[D], m, l
   unsigned long long* arrivals;   // (B*H) words: call number << 16 | splits of that call that have written their partial
   unsigned long long call;        // this call's number (unique per process): stale words of other calls read as zero arrivals
+  unsigned long long wait_ns;     // limit of each wait
+  int max_loads;                  // tiles of a split that are loaded: all of them, but for the self-test of the waits
   int* status;
 };
 int decode_splits(int D, int B, int H, int Tk);

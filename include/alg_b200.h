@@ -248,6 +248,9 @@ typedef struct {
 
 ALG_API size_t alg_decode_workspace_bytes(const alg_decode_args* args);
 ALG_API int alg_attn_decode(const alg_decode_args* args, void* stream);
+/* The same with a status word (device int, may be NULL): ALG_DEV_TIMEOUT if a wait of the kernel ran out.  With or without
+ * one, the rows of o that such a wait concerns are NaN. */
+ALG_API int alg_attn_decode_status(const alg_decode_args* args, int* status, void* stream);
 
 /* ------------------------------------------------------------------------------------
  * Fused Alg-CE head, forward, over one vocabulary shard.
@@ -519,6 +522,11 @@ ALG_API int alg_head_bwd_dz(const alg_head_bwd_args* args, void* stream);
  * NULL) the time actually spent, and the kernel returns normally. */
 ALG_API int alg_selftest_bounded_wait(int* status, unsigned long long budget_ns, unsigned long long* waited_ns,
                                       void* stream);
+/* The same for decode: a call whose kernel loads only the first `max_loads` tiles (32 keys each) of every split, so that the
+ * waits for the others run out after `budget_ns` (at most 1 s).  Calls with more tiles leave ALG_DEV_TIMEOUT in
+ * `*status` and NaN in the rows concerned. */
+ALG_API int alg_selftest_decode_timeout(const alg_decode_args* args, int max_loads, unsigned long long budget_ns, int* status,
+                                        void* stream);
 
 /* fp32 -> bf16 cast of the embedding shard (the reference casts E per call,
  * src/algebraic/kernels/fused_head.py:165; model.py:225). */

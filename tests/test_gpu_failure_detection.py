@@ -1,6 +1,6 @@
 """Failure detection without a GPU fault: a device-side wait that can never be satisfied
 runs out after its budget, the kernel reports ALG_DEV_TIMEOUT through the status word and
-returns, and the context stays usable for the next launch."""
+returns, and the context stays usable for the next launch.  A result that such a wait concerns is not a plausible one."""
 
 import pytest
 import torch
@@ -30,3 +30,27 @@ def test_bounded_wait_times_out_and_reports_status():
     # bad arguments are refused on the host
     assert lib.alg_selftest_bounded_wait(None, budget_ns, None, stream) == L.ALG_ERR_INVALID
     assert lib.alg_selftest_bounded_wait(status.data_ptr(), 5_000_000_000, None, stream) == L.ALG_ERR_INVALID
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("H,Tk,sink", [(296, 400, False), (296, 400, True), (4, 6000, True)])   # whole heads, and splits
+def test_decode_timeout_leaves_no_plausible_row(H, Tk, D, sink):
+    lib = L.load()
+    q, k, v = (torch.randn(1, H, n, D, device=DEV).bfloat16() for n in (1, Tk, Tk))
+    s = torch.randn(H, device=DEV) if sink else None
+    want = A.decode_attention(q, k, v, s)
+    o, status = torch.zeros_like(q), torch.zeros(1, dtype=torch.int32, device=DEV)
+    a = L.DecodeArgs(q=q.data_ptr(), k=k.data_ptr(), v=v.data_ptr(), o=o.data_ptr(), sink=s.data_ptr() if sink else None, B=1,
+                     H=H, Tk=Tk, D=D, n=16, c=8.0, k_stride=L.I64x3(*k.stride()[:3]), v_stride=L.I64x3(*v.stride()[:3]))
+    ws = torch.zeros(lib.alg_decode_workspace_bytes(a), dtype=torch.uint8, device=DEV)
+    a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
+    stream = torch.cuda.current_stream().cuda_stream
+    assert lib.alg_attn_decode_status(a, status.data_ptr(), stream) == L.ALG_OK
+    torch.cuda.synchronize()
+    assert int(status) == 0 and torch.equal(o, want)
+    assert lib.alg_selftest_decode_timeout(a, 1, 2_000_000, status.data_ptr(), stream) == L.ALG_OK   # one tile of each split
+    torch.cuda.synchronize()
+    assert int(status) == 1 and torch.isnan(o).all()               # ALG_DEV_TIMEOUT
+    assert torch.equal(A.decode_attention(q, k, v, s), want)
+    assert lib.alg_selftest_decode_timeout(a, 1, 2_000_000, None, stream) == L.ALG_ERR_INVALID
+    assert lib.alg_selftest_decode_timeout(a, 1, 5_000_000_000, status.data_ptr(), stream) == L.ALG_ERR_INVALID
