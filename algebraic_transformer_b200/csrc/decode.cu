@@ -22,7 +22,7 @@
 //            products: 1.1e-6 against 1.1e-7 rms of the terms' size with two keys and n = 2, 1.16e-7 now; of
 //            5.2 million outputs over 64 to 60000 keys 8935 were not the nearest bf16, 4790 with fp32 products, 4871 now.  The
 //            third part costs nothing at head_dim 64 and on single CTAs, 2 to 4 % where two CTAs of head_dim 128 share an
-//            SM: 16 x 12 x 3000 x 128 57.9 -> 59.0 us, 32 x 24 x 300 x 128 33.0 -> 34.5.)
+//            SM: 16 x 12 x 3000 x 128 57.9 -> 59.0-60.4 us, 32 x 24 x 300 x 128 33.0 -> 34.4.)
 // Single-row products leave 13 of the 16 rows idle, which costs nothing: the tensor pipe is at a few percent.
 //
 // The warp states are merged once at the end with the exact rescale (rho(m_a) rho(-m))^n.  A CTA

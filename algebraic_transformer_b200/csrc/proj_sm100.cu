@@ -413,10 +413,6 @@ proj_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
   const int rank = CG == 2 ? int(cluster_rank()) : 0;  // rank 0 issues the pair's MMAs
   constexpr uint32_t IDESC = make_idesc_bf16(BM * CG, BN, 0, 0);
   __shared__ __align__(16) float s_gain[2 * 128];      // QKV epilogue: q gains [0,128), k gains [128,256)
-  if (EPI == EPI_QKV && threadIdx.x < 2 * D) {
-    const float* g = (threadIdx.x < D) ? p.q_gain : p.k_gain;
-    s_gain[(threadIdx.x / D) * 128 + threadIdx.x % D] = (g != nullptr) ? g[threadIdx.x % D] : 1.0f;
-  }
 
   // full: bytes of both CTAs on the leader's barrier; empty, tfull: the leader's commits arrive in both CTAs;
   // tempty: every epilogue warp of both CTAs on the leader's
@@ -515,6 +511,14 @@ proj_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
     const int row_in_tile = quarter * 32 + lane;
     const uint32_t lane_sel = uint32_t(quarter * 32) << 16;
     unsigned char* stage = smem + STAGE_OFF + (warp - 2) * WARP_STAGE_BYTES;
+    if (EPI == EPI_QKV) {                                // behind griddep_wait(): the kernel ahead may be what writes the gains
+      const int i = threadIdx.x - 64;
+      if (i < 2 * D) {
+        const float* g = (i < D) ? p.q_gain : p.k_gain;
+        s_gain[(i / D) * 128 + i % D] = (g != nullptr) ? g[i % D] : 1.0f;
+      }
+      asm volatile("bar.sync 1, %0;" ::"n"(EPI_WARPS * 32) : "memory");   // the epilogue warps only; hidden behind the first products
+    }
     uint32_t tile_count = 0;
     float best_q = 0.f, best_k = 0.f, best_v = 0.f;
     bool ok = true;

@@ -1,4 +1,5 @@
-"""Calls that overlap: two streams, two threads on one stream, and a captured call whose scratch was outgrown since."""
+"""Calls that overlap: two streams, two threads on one stream, a captured call whose scratch was outgrown since, and a kernel
+that is set up while the one ahead of it still writes what it reads."""
 
 import threading
 
@@ -6,6 +7,7 @@ import pytest
 import torch
 
 import algebraic_transformer_b200 as A
+from algebraic_transformer_b200 import ops
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -88,3 +90,22 @@ def test_captured_call_outlives_larger_ones(call, make, small, large):
         torch.cuda.synchronize()
         assert all(torch.equal(x, y) for x, y in zip(out, want))
         assert all(bool((f == 255).all()) for f in filler)
+
+
+def test_gains_written_by_the_kernel_ahead():
+    """The projection kernel moves in before the kernel ahead has finished; every input has to wait for that one, gains too."""
+    M, K, H, D = 256, 128, 2, 64
+    x, w = randn((M, K), 50), randn((3 * H * D, K), 51)
+    cos, sin = A.cayley_table_geometric(D, M, device=DEV)
+    gains = torch.rand((40, D), generator=torch.Generator().manual_seed(52)).add_(0.5).to(DEV)
+    gain = torch.empty(D, device=DEV)
+
+    def project(g):
+        return ops.qkv_projection(x, w, H, M, cos.bfloat16(), sin.bfloat16(), g, g)
+    want = [project(g) for g in gains]
+    torch.cuda.synchronize()
+    got = []
+    for g in gains:
+        gain.copy_(g)
+        got.append(project(gain))
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
