@@ -23,20 +23,17 @@ from . import _lib as L
 _DTYPES = {torch.bfloat16: L.ALG_BF16, torch.float32: L.ALG_F32}
 _kept = threading.local()           # scratch of this thread, see _workspace
 _KEEP_BYTES, _KEEP_BUFFERS = 1 << 22, 32
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)       # of a device index; `torch.cuda.current_stream()`
+_capturing = getattr(torch._C, "_cuda_isCurrentStreamCapturing", None)   # builds a Stream object, 3 us a call
 
 
 def _stream():
-    """The current device's current stream as the pointer the C side takes (the raw query: `torch.cuda.current_stream()`
-    builds a Stream object, 3 us a call)."""
-    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+    """The current device's current stream as the pointer the C side takes."""
+    return _raw_stream(torch._C._cuda_getDevice())
 
 
 def _ptr(t: Optional[torch.Tensor]):
     return None if t is None else t.data_ptr()
-
-
-def _capturing() -> bool:
-    return torch._C._cuda_isCurrentStreamCapturing()
 
 
 def _workspace(device, nbytes: int, tag: str) -> torch.Tensor:
@@ -44,18 +41,16 @@ def _workspace(device, nbytes: int, tag: str) -> torch.Tensor:
     so what is kept is kept per thread and stream: calls on two streams overlap, and the launches of calls
     that two threads make on one stream mix.  A call under graph capture has a buffer of the graph's own, since a kept one can
     be replaced while the graph still replays into it.  Kept: buffers up to 4 MB, 32 a thread, for the calls
-    that are short enough to notice an allocation (1.6 us, of 15 for a decode call's host side; this costs 0.9).  They go back to
+    that are short enough to notice an allocation (1.6 us, of 15 for a decode call's host side; this costs 0.6).  They go back to
     the stream they were allocated on, with the thread at the latest."""
-    nbytes = max(int(nbytes), 256)
     if nbytes > _KEEP_BYTES or _capturing():
-        return torch.empty(nbytes, dtype=torch.uint8, device=device)
-    key = (tag, device.index, _stream())
-    kept = _kept.__dict__
+        return torch.empty(max(nbytes, 256), dtype=torch.uint8, device=device)
+    kept, key = _kept.__dict__, (tag, device.index, _raw_stream(device.index))
     buf = kept.get(key)
     if buf is None or buf.numel() < nbytes:
         if len(kept) >= _KEEP_BUFFERS:
             kept.clear()
-        buf = kept[key] = torch.empty(nbytes, dtype=torch.uint8, device=device)
+        buf = kept[key] = torch.empty(max(nbytes, 256), dtype=torch.uint8, device=device)
     return buf
 
 

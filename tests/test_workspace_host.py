@@ -14,7 +14,7 @@ CPU = torch.device("cpu")
 def place(monkeypatch):
     """The stream that is current and whether it is being captured."""
     at = {"stream": 1, "capturing": False}
-    monkeypatch.setattr(ops, "_stream", lambda: at["stream"], raising=False)
+    monkeypatch.setattr(ops, "_raw_stream", lambda index: at["stream"], raising=False)
     monkeypatch.setattr(ops, "_capturing", lambda: at["capturing"], raising=False)
     monkeypatch.setattr(ops, "_kept", threading.local(), raising=False)
     return at
