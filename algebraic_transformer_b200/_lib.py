@@ -154,6 +154,7 @@ SYMBOLS = {
     "alg_resid_proj_fwd": (C.c_int, [C.POINTER(ResidProjArgs), C.c_void_p]),
     "alg_resid_proj_ss_slots": (C.c_int, [C.c_int, C.c_int]),
     "alg_row_sumsq": (C.c_int, [C.c_void_p, C.c_int64, C.c_int, C.c_int64, C.c_void_p, C.c_void_p]),
+    "alg_gemm_plan": (C.c_int, [C.c_int] * 5 + [C.POINTER(C.c_int)] * 3),
     "alg_selftest_decode_timeout": (C.c_int, [C.POINTER(DecodeArgs), C.c_int, C.c_ulonglong, C.c_void_p, C.c_void_p]),
     "alg_selftest_bounded_wait": (C.c_int, [C.c_void_p, C.c_ulonglong, C.c_void_p, C.c_void_p]),
     "alg_rms_norm_fwd":(C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int, C.c_float, C.c_void_p]),

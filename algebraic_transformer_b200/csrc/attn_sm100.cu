@@ -1247,7 +1247,8 @@ int launch_kernel(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMa
 // Items of one query tile or of two.  Two tiles share their K and V tiles and keep the pipes busier, but a step of
 // both takes longer than a step of one: where the longest item sets the time, one tile ends sooner.  The estimate is
 // the longest CTA's steps (the longest item, or an even share and one for the uneven deal) times the time of a step, one
-// tile's being 0.75 to 0.9 of two tiles'.  Measured, two -> one: (1,12,613,64) 14.8 -> 10.9 us, (1,12,2048,64) 31.9 -> 24.6,
+// tile's being 0.75 to 0.9 of two tiles' and counted as 0.9 (head_dim 128: 0.95), at the upper end, so that near ties stay
+// with two.  Measured, two -> one: (1,12,613,64) 14.8 -> 10.9 us, (1,12,2048,64) 31.9 -> 24.6,
 // (1,16,613,128) 17.5 -> 14.3, (1,16,2048,128) 35.9 -> 33.3; (2,12,2048,64) 32.0 -> 38.2, (16,12,1024,64) 61 -> 84.
 template <int D>
 bool single_tiles(int units, int T, int grid) {

@@ -412,6 +412,18 @@ int alg_resid_proj_ss_slots(int M, int N) {
   return 2 * ((N + bn - 1) / bn);
 }
 
+int alg_gemm_plan(int op, int M, int K, int N, int D, int* tile_width, int* ctas, int* k_parts) {
+  if (op < 0 || op > 4 || M < 1 || N < 1 || K < 64 || K % 64 != 0) {
+    set_error("gemm_plan: op 0 to 4, positive extents, K a multiple of 64");
+    return ALG_ERR_INVALID;
+  }
+  const ProjPlan pl = op == 4 ? ProjPlan{256, head_tcgen05_ctas(M, N, K), 1} : proj_plan(op, M, K, N, D);
+  if (tile_width != nullptr) *tile_width = pl.bn;
+  if (ctas != nullptr) *ctas = pl.cg;
+  if (k_parts != nullptr) *k_parts = pl.k_parts;
+  return ALG_OK;
+}
+
 int alg_resid_proj_fwd(const alg_resid_proj_args* a, void* stream_) {
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   if (a == nullptr || a->x == nullptr || a->w == nullptr || a->resid == nullptr || a->out == nullptr) {

@@ -9,6 +9,9 @@
 //                      columns), w = rho_fast(min(z/c, clamp))^n, row sums, target pick —
 //                      while the MMA warp already fills the other TMEM buffer
 //
+// Where pair_size (launchers.h) says so, two CTAs of a cluster share a 256x256 tile: each loads its 128 rows of h and half of
+// the tile's rows of E and keeps its 128 accumulator rows, and the leader issues the products of both (cta_group::2).
+//
 // Logits never leave the SM.  A CTA walks "units" = (128-token block, run of vocabulary
 // tiles); per unit each epilogue thread writes one partial (l, zt) for its row and column
 // half, and head_reduce adds the partials in a fixed order (deterministic results).
@@ -309,9 +312,14 @@ int head_tcgen05_splits(int N, int V_local) {
   return 2 * make_plan(N, V_local).S;
 }
 
+int head_tcgen05_ctas(int N, int V_local, int d) {
+  const Plan pl = make_plan(N, V_local);
+  return pair_size(pl.row_blocks, pl.S, pl.tps * (d / BK));
+}
+
 int launch_head_tcgen05(const HeadParams& p, cudaStream_t stream) {
   const Plan pl = make_plan(p.N, p.V_local);
-  const int cg = pair_size(pl.row_blocks, pl.S, pl.tps * (p.d / BK));
+  const int cg = head_tcgen05_ctas(p.N, p.V_local, p.d);
   CUtensorMap tm_h, tm_e;
   {
     const uint64_t dims[2] = {uint64_t(p.d), uint64_t(p.N)};

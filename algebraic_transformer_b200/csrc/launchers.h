@@ -202,6 +202,8 @@ struct ProjParams {
 };
 int launch_proj(const ProjParams& p, const void* x, const void* w, int epi, cudaStream_t stream);   // epi 0 QKV, 1 GLU, 2 head dz, 3 residual
 int proj_resid_tile_width(int M, int N);
+struct ProjPlan { int bn, cg, k_parts; };   // tile width, CTAs that share an accumulator tile, parts of K
+ProjPlan proj_plan(int epi, int M, int K, int N, int D);
 // prefill_ops.cu
 int launch_row_sumsq(const void* x, int64_t rows, int d, int64_t ld, float* ss_out, cudaStream_t stream);
 
@@ -251,6 +253,7 @@ int launch_head_mma(const HeadParams& p, cudaStream_t stream);
 bool head_tcgen05_supports(const HeadParams& p);
 int head_tcgen05_splits(int N, int V_local);
 int launch_head_tcgen05(const HeadParams& p, cudaStream_t stream);
+int head_tcgen05_ctas(int N, int V_local, int d);   // CTAs that share an accumulator tile
 int launch_head_reduce(const HeadParams& p, cudaStream_t stream);
 int launch_head_finalize(const float* l, const float* zt, int N, int log2n, float inv_c, float clamp,
                          float* pt, float* nll, float* obj, float* block_sums, unsigned* ticket,

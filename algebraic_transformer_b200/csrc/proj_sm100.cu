@@ -26,7 +26,9 @@
 // feeds a shared-memory ring with TMA (128x64 activation tiles, 256x64 weight tiles,
 // 128-byte swizzle), warp 1 issues tcgen05.mma 128x256x16 into one of two 256-column
 // TMEM accumulators, warps 2..9 drain the finished accumulator (thread = row) while the other
-// one fills.  The epilogues keep values as packed bf16 pairs wherever the reference's
+// one fills.  Large problems run on CTA pairs (cta_group::2, pair_size in launchers.h): 256 x 256 tiles, each CTA
+// loading its 128 activation rows and half of the weight rows and keeping its 128 accumulator rows, the leader issuing
+// for both.  Small ones take 128-wide tiles, and the residual GEMM of few rows splits K over a cluster (proj_plan).  The epilogues keep values as packed bf16 pairs wherever the reference's
 // arithmetic is bf16 (one conversion or one HMUL2/HADD2 per two elements) and keep the next
 // tensor-memory load in flight while the current chunk is worked on: with K of only 768..1536
 // the accumulator turns over every few microseconds and the epilogue is what has to keep up.
@@ -813,9 +815,31 @@ int proj_resid_tile_width(int M, int N) {
   return cost_narrow < cost_wide ? 128 : 256;
 }
 
+// Tile, CTAs that share one, and parts of K over a cluster for a GEMM (M, K) x (N, K)^T.
+ProjPlan proj_plan(int epi, int M, int K, int N, int D) {
+  // QKV (head_dim 64) and GLU: narrow tiles only where they are one round - their epilogues weigh more than the residual's
+  // (GLU 1024 x 1024 x 2688, 2 wide rounds or 3 narrow ones: 16.5 and 20.0 us; QKV 613 x 768, one of either: 10.0 and 7.9)
+  ProjPlan pl{BN_MAX, 1, 1};
+  const int row_blocks = (M + BM - 1) / BM, steps = K / BK;
+  if (epi == EPI_RESID) pl.bn = proj_resid_tile_width(M, N);
+  else if ((epi == EPI_GLU || (epi == EPI_QKV && D == 64)) && row_blocks * ((N + 127) / 128) <= sm_count()) pl.bn = 128;
+  if (pl.bn == BN_MAX) pl.cg = pair_size(row_blocks, (N + pl.bn - 1) / pl.bn, steps);
+  if (epi == EPI_RESID && pl.bn == 128) {
+    // K over four CTAs from 16 ring steps on, over two from 32, where the chip has room (613 rows, K = 2048: 11.6 us whole, 10.1
+    // over two, 8.3 over four; 64 rows 11.3 and 7.5; 1024 x 2688 x 1024 14.3 and 12.0 over two).  Shorter K do not pay for
+    // the exchange (613 x 768 x 768, 12 steps: 6.7 whole, 7.7 and 6.9; 1024 x 1024 x 1024, 16 steps: 7.9 and 8.5 over two).
+    const int tiles = row_blocks * ((N + 127) / 128);
+    if (steps >= 16 && tiles * 4 <= sm_count()) pl.k_parts = 4;
+    else if (steps >= 32 && tiles * 2 <= sm_count()) pl.k_parts = 2;
+  }
+  return pl;
+}
+
 int launch_proj(const ProjParams& params, const void* x, const void* w, int epi, cudaStream_t stream) {
   ProjParams p = params;
   if (p.M == 0) return ALG_OK;
+  const ProjPlan pl = proj_plan(epi, p.M, p.K, p.N, p.D);
+  const int bn = pl.bn, cg = pl.cg;
   CUtensorMap tm_x, tm_w;
   {
     const uint64_t dims[2] = {uint64_t(p.K), uint64_t(p.M)};
@@ -823,12 +847,6 @@ int launch_proj(const ProjParams& params, const void* x, const void* w, int epi,
     const uint32_t box[2] = {BK, BM};
     if (int rc = make_tmap_bf16(&tm_x, x, 2, dims, strides, box, true)) return rc;
   }
-  // QKV (head_dim 64) and GLU: narrow tiles only where they are one round - their epilogues weigh more than the residual's
-  // (GLU 1024 x 1024 x 2688, 2 wide rounds or 3 narrow ones: 16.5 and 20.0 us; QKV 613 x 768, one of either: 10.0 and 7.9)
-  int bn = BN_MAX;
-  if (epi == EPI_RESID) bn = proj_resid_tile_width(p.M, p.N);
-  else if ((epi == EPI_GLU || (epi == EPI_QKV && p.D == 64)) && ((p.M + BM - 1) / BM) * ((p.N + 127) / 128) <= sm_count()) bn = 128;
-  const int cg = bn == BN_MAX ? pair_size((p.M + BM - 1) / BM, (p.N + bn - 1) / bn, p.K / BK) : 1;
   {
     const uint64_t dims[2] = {uint64_t(p.K), uint64_t(p.N)};
     const uint64_t strides[1] = {uint64_t(p.K)};
@@ -840,14 +858,8 @@ int launch_proj(const ProjParams& params, const void* x, const void* w, int epi,
   // one round: the next kernel's CTAs set up on the SMs left free (hidden states of the 125M model, 613 tokens: 653 -> 604 us;
   // with more rounds they would sit beside running ones)
   p.announce = tiles <= places;
-  if (epi == EPI_RESID && bn == 128) {
-    // K over four CTAs from 16 ring steps on, over two from 32, where the chip has room (613 rows, K = 2048: 11.6 us whole, 10.1
-    // over two, 8.3 over four; 64 rows 11.3 and 7.5; 1024 x 2688 x 1024 14.3 and 12.0 over two).  Shorter K do not pay for
-    // the exchange (613 x 768 x 768, 12 steps: 6.7 whole, 7.7 and 6.9; 1024 x 1024 x 1024, 16 steps: 7.9 and 8.5 over two).
-    const int steps = p.K / BK;
-    if (steps >= 16 && tiles * 4 <= places) return launch_split<4>(tm_x, tm_w, p, tiles, stream);
-    if (steps >= 32 && tiles * 2 <= places) return launch_split<2>(tm_x, tm_w, p, tiles, stream);
-  }
+  if (pl.k_parts == 4) return launch_split<4>(tm_x, tm_w, p, tiles, stream);
+  if (pl.k_parts == 2) return launch_split<2>(tm_x, tm_w, p, tiles, stream);
   const int grid = (tiles < places ? tiles : places) * cg;
   if (cg == 2) return launch_tile<256, 2>(tm_x, tm_w, p, epi, grid, stream);
   return bn == 128 ? launch_tile<128, 1>(tm_x, tm_w, p, epi, grid, stream) : launch_tile<256, 1>(tm_x, tm_w, p, epi, grid, stream);

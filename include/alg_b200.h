@@ -515,6 +515,12 @@ typedef struct {
 } alg_head_bwd_args;
 ALG_API int alg_head_bwd_dz(const alg_head_bwd_args* args, void* stream);
 
+/* How the GEMM kernels would cut a problem on the current device: CTAs that share an accumulator tile (1, or a pair) in
+ * `*ctas`, the tile's width in `*tile_width`, the parts of K in `*k_parts` (each may be NULL).  op 0: alg_qkv_proj_fwd (M, K = d,
+ * N = 3 H D, D); 1: alg_glu_proj_fwd (K = d, N = 2 f); 2: alg_head_bwd_dz (N = V_local); 3: alg_resid_proj_fwd; 4: the tcgen05
+ * form of alg_head_fwd (M = N_tokens, K = d, N = V_local).  D counts for op 0 only. */
+ALG_API int alg_gemm_plan(int op, int M, int K, int N, int D, int* tile_width, int* ctas, int* k_parts);
+
 /* Failure-detection self-test (no counterpart in the reference).  Launches a one-CTA kernel
  * whose threads wait, through the same bounded-wait helper every TMA/tcgen05 kernel here
  * uses, on a barrier that is never signalled.  After `budget_ns` (at most 1 s) the wait
