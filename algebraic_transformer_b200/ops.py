@@ -41,11 +41,13 @@ def _workspace(device, nbytes: int, tag: str) -> torch.Tensor:
     so what is kept is kept per thread and stream: calls on two streams overlap, and the launches of calls
     that two threads make on one stream mix.  A call under graph capture has a buffer of the graph's own, since a kept one can
     be replaced while the graph still replays into it.  Kept: buffers up to 4 MB, 32 a thread, for the calls
-    that are short enough to notice an allocation (1.6 us, of 15 for a decode call's host side; this costs 0.6).  They go back to
+    that are short enough to notice an allocation (1.6 us, of 15 for a decode call's host side; this costs 0.3 to 0.6).  They go back to
     the stream they were allocated on, with the thread at the latest."""
-    if nbytes > _KEEP_BYTES or _capturing():
+    index = device.index
+    stream = _raw_stream(index)
+    if nbytes > _KEEP_BYTES or (stream and _capturing()):   # stream 0, the default one, cannot be captured
         return torch.empty(max(nbytes, 256), dtype=torch.uint8, device=device)
-    kept, key = _kept.__dict__, (tag, device.index, _raw_stream(device.index))
+    kept, key = _kept.__dict__, (tag, index, stream)
     buf = kept.get(key)
     if buf is None or buf.numel() < nbytes:
         if len(kept) >= _KEEP_BUFFERS:
