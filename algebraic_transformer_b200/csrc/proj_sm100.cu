@@ -803,15 +803,17 @@ int launch_split(const CUtensorMap& tm_x, const CUtensorMap& tm_w, const ProjPar
 
 }  // namespace
 
-// The residual GEMM's tiles are 128 x 256 unless 128 x 128 ones spread better over the SMs (few rows: a short prompt, or a
-// rank's share of a batch split over many GPUs).  Cost model: rounds of tiles per CTA times the time of
-// one tile.  A narrow tile takes a little more than half of a wide one while its rows come from L2; from HBM about
-// two thirds, its operands being 32 KB per 256 cycles of products (K = 2688, N = 1024: 8192 rows, 44 MB, 34.0 us narrow
-// and 37.8 wide; 16384 rows 94 us in 7 narrow rounds and 70 in 4 wide ones).
+// The residual GEMM's tiles are 128 x 256 unless 128 x 128 ones take so many fewer rounds that they end sooner (few rows: a
+// short prompt, or a rank's share of a batch split over many GPUs).  A round of narrow tiles takes 0.58 to 0.68 of a round
+// of wide ones at K = 768, where the epilogue is a good part of it, 0.71 to 0.85 at 2048 and up to 0.88 at 4096, where
+// their operand traffic is (32 KB per 256 cycles of products, 48 KB per 512); the rows make no difference (6016 to 18432).
+// The rule may not look at K, since the row statistic's slots follow from rows and columns: three narrow rounds for
+// two wide ones are about even at K = 768 (8192 x 768 x 768 17.5 us narrow, 18.3 wide) and lose from 2048 on (8192 x 2048 x 768
+// 34.3 and 28.2, 5600 x 2688 x 1024 42.6 and 33.9), five for three lose everywhere (14080 x 768 x 768 26.4 and 24.2).
 int proj_resid_tile_width(int M, int N) {
   const int sms = sm_count(), mt = (M + BM - 1) / BM;
   const int wide = mt * ((N + 255) / 256), narrow = mt * ((N + 127) / 128);
-  const double cost_wide = double((wide + sms - 1) / sms), cost_narrow = (M <= 8192 ? 0.55 : 0.67) * double((narrow + sms - 1) / sms);
+  const double cost_wide = double((wide + sms - 1) / sms), cost_narrow = 0.67 * double((narrow + sms - 1) / sms);
   return cost_narrow < cost_wide ? 128 : 256;
 }
 
