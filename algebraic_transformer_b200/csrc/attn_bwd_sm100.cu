@@ -35,11 +35,12 @@
 //   head_dim 64   BS = 64: a CTA then needs 256 tensor-memory columns and 98 KB of shared memory, and TWO
 //                 CTAs share an SM, so one computes while the other waits, loads or stores.  The 64-wide
 //                 score products take nearly as long as 128-wide ones; the overlap is worth more.
-// Measured (CUDA-graph replay, delta kernel included; before = 128-wide steps, 8 warps of 64 columns, one launch
-// per kind, mma.sync kernels for lengths off 128): (16,12,1024,64) 272 -> 174 us, (8,16,2048,64) 531 -> 366,
-// (1,16,8192,64) 786 -> 625, (1,16,8192,128) 1090 -> 960, (2,16,1837,128) 563 -> 146, (5,12,489,64) 85 -> 28.
-// BS = 128 with one CTA at head_dim 64: 245 / 496 us for the first two.  Two warp sets on alternate 64-wide steps in
-// one CTA (257 us; head_dim 128: 1036): 64-wide score products cost the tensor pipe what 128-wide ones do.
+// Measured (CUDA-graph replay over several sets of inputs, delta kernel included; before = 128-wide steps, 8 warps of 64
+// columns, one launch per kind, mma.sync kernels for lengths off 128): (16,12,1024,64) 317 -> 181 us, (8,16,2048,64) 578 -> 384,
+// (1,16,8192,64) 808 -> 620, (1,16,8192,128) 1017 -> 900-920, (2,16,1837,128) 591 -> 142, (5,12,489,64) 102 -> 35.
+// Other forms of this one, where (16,12,1024,64) took 174 us and (8,16,2048,64) 366 on one set of inputs: BS = 128 with one CTA at
+// head_dim 64 245 / 496 us; two warp sets on alternate 64-wide steps in one CTA 257 us (head_dim 128: 1036 against 960), since
+// 64-wide score products cost the tensor pipe what 128-wide ones do.
 //
 // Lengths off the tile: TMA fills rows past the end with zeros.  Keys past the end lie above the
 // diagonal of every real query; queries past the end get statistic and delta 0, hence weight 0; rows past

@@ -441,6 +441,14 @@ proj_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
   // stream; from here on its results are complete.
   griddep_wait();
   if (p.announce) griddep_launch();
+  if (EPI == EPI_QKV && threadIdx.x >= 64) {           // behind the wait: the kernel ahead may be what writes the gains
+    const int i = threadIdx.x - 64;
+    if (i < 2 * D) {
+      const float* g = (i < D) ? p.q_gain : p.k_gain;
+      s_gain[(i / D) * 128 + i % D] = (g != nullptr) ? g[i % D] : 1.0f;
+    }
+    asm volatile("bar.sync 1, %0;" ::"n"(EPI_WARPS * 32) : "memory");   // the epilogue warps only; hidden behind the first products
+  }
   const uint32_t tmem_base = ctl->tmem_base;
   const BoundedWait bw{&ctl->abort_flag, 1000000000ull};
   const int tiles_n = (p.N + BN - 1) / BN;
@@ -513,14 +521,6 @@ proj_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
     const int row_in_tile = quarter * 32 + lane;
     const uint32_t lane_sel = uint32_t(quarter * 32) << 16;
     unsigned char* stage = smem + STAGE_OFF + (warp - 2) * WARP_STAGE_BYTES;
-    if (EPI == EPI_QKV) {                                // behind griddep_wait(): the kernel ahead may be what writes the gains
-      const int i = threadIdx.x - 64;
-      if (i < 2 * D) {
-        const float* g = (i < D) ? p.q_gain : p.k_gain;
-        s_gain[(i / D) * 128 + i % D] = (g != nullptr) ? g[i % D] : 1.0f;
-      }
-      asm volatile("bar.sync 1, %0;" ::"n"(EPI_WARPS * 32) : "memory");   // the epilogue warps only; hidden behind the first products
-    }
     uint32_t tile_count = 0;
     float best_q = 0.f, best_k = 0.f, best_v = 0.f;
     bool ok = true;

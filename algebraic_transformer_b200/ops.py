@@ -22,7 +22,7 @@ from . import _lib as L
 
 _DTYPES = {torch.bfloat16: L.ALG_BF16, torch.float32: L.ALG_F32}
 _kept = threading.local()           # scratch of this thread, see _workspace
-_KEEP_BYTES, _KEEP_BUFFERS = 1 << 22, 32
+_KEEP_BYTES, _KEEP_BUFFERS, _KEEP_TOTAL = 1 << 25, 32, 1 << 28
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)       # of a device index; `torch.cuda.current_stream()`
 _capturing = getattr(torch._C, "_cuda_isCurrentStreamCapturing", None)   # builds a Stream object, 3 us a call
 
@@ -40,9 +40,9 @@ def _workspace(device, nbytes: int, tag: str) -> torch.Tensor:
     """Scratch for one call on the current stream.  Two calls may use the same buffer only if one comes after the other,
     so what is kept is kept per thread and stream: calls on two streams overlap, and the launches of calls
     that two threads make on one stream mix.  A call under graph capture has a buffer of the graph's own, since a kept one can
-    be replaced while the graph still replays into it.  Kept: buffers up to 4 MB, 32 a thread, for the calls
-    that are short enough to notice an allocation (1.6 us, of 15 for a decode call's host side; this costs 0.3 to 0.6).  They go back to
-    the stream they were allocated on, with the thread at the latest."""
+    be replaced while the graph still replays into it.  Kept: buffers up to 32 MB, 32 of them and 256 MB a thread, for the
+    calls that are short enough to notice an allocation (1.6 to 2.4 us, of 15 for a decode call's host side; this costs 0.3
+    to 0.6).  They go back to the stream they were allocated on, with the thread at the latest."""
     index = device.index
     stream = _raw_stream(index)
     if nbytes > _KEEP_BYTES or (stream and _capturing()):   # stream 0, the default one, cannot be captured
@@ -50,7 +50,7 @@ def _workspace(device, nbytes: int, tag: str) -> torch.Tensor:
     kept, key = _kept.__dict__, (tag, index, stream)
     buf = kept.get(key)
     if buf is None or buf.numel() < nbytes:
-        if len(kept) >= _KEEP_BUFFERS:
+        if len(kept) >= _KEEP_BUFFERS or sum(b.numel() for b in kept.values()) + nbytes > _KEEP_TOTAL:
             kept.clear()
         buf = kept[key] = torch.empty(max(nbytes, 256), dtype=torch.uint8, device=device)
     return buf

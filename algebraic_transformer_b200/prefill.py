@@ -133,8 +133,8 @@ class Prefill:
         # `fused_norm`: the block norms as row scales inside the projections and the residual adds inside
         # the out- and down-projection (five GEMM launches per block, no stand-alone norm).  None = wherever the
         # projections are fused.  Measured against stand-alone norms + library GEMMs with the residual in
-        # their epilogue, hidden states of one call: 125M 16384 tokens 3.24 ms against 3.34, 350M 16384 tokens 10.5
-        # against 11.0, 1B 16384 tokens 29-31 against 32; 3-4 % faster up to 4096 tokens.
+        # their epilogue, hidden states of one call of 16384 tokens: 125M 3.0-3.5 ms against 3.4-3.7, 350M 11.4-11.7
+        # against 12.5-12.7, 1B 30.7-31.1 against 32.2-32.9; 3-4 % faster up to 4096 tokens.
         if fused_norm and not self.fused_proj:
             raise ValueError("fused_norm needs the fused projections")
         self.fused_norm = fused_norm if (fused_norm is None or not self.fused_proj) else bool(fused_norm)

@@ -62,3 +62,7 @@ def test_what_is_kept_is_bounded(place):
         place["stream"] = stream
         take()
         assert len(ops._kept.__dict__) <= ops._KEEP_BUFFERS
+    for stream in range(20):
+        place["stream"] = stream
+        take(ops._KEEP_BYTES)
+        assert sum(b.numel() for b in ops._kept.__dict__.values()) <= ops._KEEP_TOTAL
