@@ -413,8 +413,8 @@ int alg_resid_proj_ss_slots(int M, int N) {
 }
 
 int alg_gemm_plan(int op, int M, int K, int N, int D, int* tile_width, int* ctas, int* k_parts) {
-  if (op < 0 || op > 4 || M < 1 || N < 1 || K < 64 || K % 64 != 0) {
-    set_error("gemm_plan: op 0 to 4, positive extents, K a multiple of 64");
+  if (op < 0 || op > 4 || M < 1 || N < 1 || K < 64 || K % 64 != 0 || int64_t(M) * N > (int64_t(1) << 44)) {
+    set_error("gemm_plan: op 0 to 4, positive extents that memory holds, K a multiple of 64");
     return ALG_ERR_INVALID;
   }
   const ProjPlan pl = op == 4 ? ProjPlan{256, head_tcgen05_ctas(M, N, K), 1} : proj_plan(op, M, K, N, D);

@@ -38,4 +38,5 @@ def test_pairs_and_parts():
     assert plan(RESID, 613, 2048, 768) == (128, 1, 4) and plan(RESID, 16384, 2048, 768) == (256, 2, 1)
     assert plan(HEAD, 8192, 768, 50304)[1] == 2 and plan(DZ, 8192, 768, 50304) == (256, 2, 1)
     assert L.load().alg_gemm_plan(5, 128, 64, 128, 64, None, None, None) == L.ALG_ERR_INVALID
+    assert L.load().alg_gemm_plan(RESID, 2**31 - 1, 64, 2**31 - 1, 64, None, None, None) == L.ALG_ERR_INVALID
     assert L.load().alg_gemm_plan(RESID, 128, 65, 128, 64, None, None, None) == L.ALG_ERR_INVALID
